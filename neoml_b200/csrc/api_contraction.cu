@@ -106,6 +106,17 @@ size_t prepared_filter_floats(long long k, long long r, long long s, long long c
 	return static_cast<size_t>((k * r * s * c + 3) / 4 * 4);
 }
 
+// Whether a launch of this many 128-row tiles, n columns and depth k goes to the fp16 kernel (3xTF32 accuracy,
+// contraction_split.cu) when its second operand is prepared: from the tile count on that no longer splits K, i.e. where
+// throughput and not the length of one tile's K loop decides (below it the TF32 kernel with split K stays), and from five
+// K blocks on (a shorter loop is hidden behind its epilogue; ResNet-50 at batch 256, TF32 against fp16 kernel: K = 64 and
+// 128 with residual 355 / 430 us and 197 / 239, K = 256 158 / 150, K = 1152 284 / 195).
+bool split_form_pays(long long mTiles, long long n, long long k, long long batch)
+{
+	const int width = contraction_tile_width(static_cast<int>(n));
+	return k > 128 && mTiles * ((n + width - 1) / width) * batch > SPLIT_TILES_MAX;
+}
+
 // Row-window form of a convolution with few channels (the network stem): the image is copied once with its spatial
 // zero padding and its channels widened to a multiple of four, so that the S taps of one filter row are ONE contiguous
 // run of at most 32 floats per output position; the filter rows are widened to 32 floats with zeros.
@@ -176,6 +187,28 @@ void prepare_window_filter(void* stream, const nb200_conv_desc* d, const WindowP
 	count_launch(2);
 }
 
+bool split_form_pays(const nb200_conv_desc* d, bool window)
+{
+	if(d->batch <= 0 || d->ho <= 0 || d->wo <= 0 || d->k <= 0) return false;
+	const long long rows = static_cast<long long>(d->batch) * d->ho * d->wo;
+	return rows >= PREPARE_B_MIN_ROWS && split_form_pays(window ? static_cast<long long>(d->batch) * d->ho : (rows + 127) / 128,
+		d->k, window ? d->r * 32LL : static_cast<long long>(d->r) * d->s * d->c, 1);
+}
+
+// floats of a matrix product's second operand as it lies in memory, rounded up: where the split form begins in a
+// prepared operand
+size_t prepared_span(int n, int k, int ldb)
+{
+	return (static_cast<size_t>(n - 1) * ldb + k + 3) / 4 * 4;
+}
+
+void set_split_operand(ContractionParams& p, const float* form, long long rows, long long k)
+{
+	p.bSplit = form;
+	p.bScale = form + rows * ((k + 31) / 32 * 32);
+	p.b_ready = 1;
+}
+
 bool wants_channel_padding(const nb200_conv_desc* d)
 {
 	const bool pointwise = d->r == 1 && d->s == 1 && d->pad_h == 0 && d->pad_w == 0 && d->stride_h == 1 && d->stride_w == 1;
@@ -192,6 +225,13 @@ size_t convolution_scratch_floats(const nb200_conv_desc* d, bool withSplitRoom)
 	WindowPlan win;
 	if(plan_row_window(d, &win)) return win.imageFloats + 2 * win.filterFloats + 16;
 	size_t floats = prepared_filter_floats(d->k, d->r, d->s, static_cast<long long>(c4)) + 8;
+	// (withSplitRoom: also what is only wanted -- a caller with less room gets the forms that fit)
+	nb200_conv_desc padded = *d;
+	padded.c = static_cast<int>(c4);
+	if(withSplitRoom && (split_form_pays(d, false) || split_form_pays(&padded, false))) {
+		const size_t split = split_operand_floats(d->k, static_cast<long long>(d->r) * d->s * c4) + 8;
+		if(split > floats) floats = split;
+	}
 	if(wants_channel_padding(d)) floats += (static_cast<size_t>(d->batch) * d->h * d->w + static_cast<size_t>(d->k) * d->r * d->s) * c4 + 8;
 	// last, so that a caller with less room loses only the split
 	if(withSplitRoom && d->ho > 0 && d->wo > 0) {
@@ -270,7 +310,14 @@ size_t nb200_matrix_product_scratch_floats(int batch, int m, int n, int k, int l
 	if(batch <= 0 || m <= 0 || n <= 0 || k <= 0 || ldb < k) return 0;
 	size_t floats = 0;
 	// the split second operand pays when it is reused by several row tiles
-	if(m >= PREPARE_B_MIN_ROWS) floats += (static_cast<size_t>(batch) * n * ldb + 3) / 4 * 4 + 8;
+	if(m >= PREPARE_B_MIN_ROWS) {
+		floats += (static_cast<size_t>(batch) * n * ldb + 3) / 4 * 4;
+		if(split_form_pays((static_cast<long long>(m) + 127) / 128, n, k, batch)) {
+			const size_t split = split_operand_floats(static_cast<long long>(batch) * n, k);
+			if(split > floats) floats = split;
+		}
+		floats += 8;
+	}
 	if(batch == 1) floats += split_scratch_floats(m, n, k);
 	return floats;
 }
@@ -300,9 +347,20 @@ static int matrix_product(void* stream, int batch, const float* a, int m, int k,
 	const bool wanted = m >= PREPARE_B_MIN_ROWS;
 	const bool given = wanted && prepared != nullptr && batch == 1 && aligned16(prepared);
 	const bool prepare = wanted && !given && rest != nullptr;
-	if(given) {
+	const bool split = precision == NB200_PREC_3XTF32 && split_form_pays((static_cast<long long>(m) + 127) / 128, n, k, batch);
+	if(given && split) {
+		// both forms are in the prepared operand, which serves products of any height
+		set_split_operand(p, prepared + prepared_span(n, k, ldb), n, k);
+	} else if(given) {
 		if(precision == NB200_PREC_3XTF32) p.Blo = prepared; else p.B = prepared;
 		p.b_ready = 1;
+	} else if(prepare && split) {
+		if(device_status_word() == nullptr) return NB200_ENODEVICE;
+		// the rows of all batch entries are one matrix: an entry is n rows of ldb floats
+		const long long rows = static_cast<long long>(batch) * n;
+		const int rc = split_operand(b, rows, ldb, k, rest, as_stream(stream));
+		if(rc != NB200_OK) return rc;
+		set_split_operand(p, rest, rows, k);
 	} else if(prepare) {
 		// one pass over the second operand as it lies in memory (the floats between its rows, if any, are carried along)
 		if(device_status_word() == nullptr) return NB200_ENODEVICE;
@@ -323,7 +381,7 @@ static int matrix_product(void* stream, int batch, const float* a, int m, int k,
 	const int rc = run(p, batch, stream, precision);
 	if(rc != NB200_EINVAL || !(prepare || given)) return rc;
 	// the launcher could not describe an operand to TMA after all: in-kernel conversion, unsplit
-	p.B = b; p.Blo = nullptr; p.b_ready = 0; p.splitScratch = nullptr;
+	p.B = b; p.Blo = nullptr; p.bSplit = nullptr; p.b_ready = 0; p.splitScratch = nullptr;
 	return run(p, batch, stream, precision);
 }
 
@@ -336,7 +394,7 @@ int nb200_multiply_matrix_by_transposed_matrix_with_scratch(void* stream, int ba
 size_t nb200_matrix_product_prepared_floats(int m, int n, int k, int ldb)
 {
 	if(m < PREPARE_B_MIN_ROWS || n <= 0 || k <= 0 || ldb < k) return 0;
-	return (static_cast<size_t>(n - 1) * ldb + k + 3) / 4 * 4;
+	return prepared_span(n, k, ldb) + split_operand_floats(n, k);
 }
 
 int nb200_matrix_product_prepare_second(void* stream, const float* b, int n, int k, int ldb, float* prepared, int precision)
@@ -348,6 +406,10 @@ int nb200_matrix_product_prepare_second(void* stream, const float* b, int n, int
 	prepare_filter_kernel<<<grid_for(span, 256, 8), 256, 0, as_stream(stream)>>>(b, prepared, span,
 		precision == NB200_PREC_3XTF32 ? 0 : 1);
 	count_launch(1);
+	// the split form for tall products; it is read only where the rows are 16-byte aligned
+	if(precision == NB200_PREC_3XTF32 && vec_ok(b, ldb, 0)) {
+		return split_operand(b, n, ldb, k, prepared + prepared_span(n, k, ldb), as_stream(stream));
+	}
 	return check_launch();
 }
 
@@ -387,12 +449,12 @@ size_t nb200_blob_convolution_prepared_filter_floats(const nb200_conv_desc* d)
 {
 	if(d == nullptr || d->c <= 0 || d->k <= 0 || d->r <= 0 || d->s <= 0 || d->ho <= 0 || d->wo <= 0 || d->batch <= 0) return 0;
 	WindowPlan win;
-	if(plan_row_window(d, &win)) return 2 * win.filterFloats;
+	if(plan_row_window(d, &win)) return 2 * win.filterFloats + split_operand_floats(d->k, d->r * 32LL);
 	const bool pointwise = d->r == 1 && d->s == 1 && d->pad_h == 0 && d->pad_w == 0 && d->stride_h == 1 && d->stride_w == 1;
 	const long long kk = static_cast<long long>(d->r) * d->s * d->c;
 	const bool tmaShape = (pointwise ? d->c % 4 == 0 : d->c % 32 == 0) && kk % 4 == 0;
 	if(!tmaShape || static_cast<long long>(d->batch) * d->ho * d->wo < PREPARE_B_MIN_ROWS) return 0;
-	return prepared_filter_floats(d->k, d->r, d->s, d->c);
+	return prepared_filter_floats(d->k, d->r, d->s, d->c) + split_operand_floats(d->k, kk);
 }
 
 int nb200_blob_convolution_prepare_filter(void* stream, const nb200_conv_desc* d, const float* filter, float* prepared,
@@ -408,11 +470,19 @@ int nb200_blob_convolution_prepare_filter(void* stream, const nb200_conv_desc* d
 	WindowPlan win;
 	if(plan_row_window(d, &win)) {
 		prepare_window_filter(stream, d, &win, filter, prepared, precision);
+		// both forms: the prepared filter serves batches on either side of the line between the kernels
+		if(precision == NB200_PREC_3XTF32) {
+			return split_window_filter(filter, d->k, d->r, d->s, d->c, win.c4, prepared + 2 * win.filterFloats, as_stream(stream));
+		}
 	} else {
 		const long long n = static_cast<long long>(d->k) * d->r * d->s * d->c;
 		prepare_filter_kernel<<<grid_for(n, 256, 8), 256, 0, as_stream(stream)>>>(filter, prepared, n,
 			precision == NB200_PREC_3XTF32 ? 0 : 1);
 		count_launch(1);
+		const int kk = d->r * d->s * d->c;
+		if(precision == NB200_PREC_3XTF32 && vec_ok(filter, kk, 0)) {
+			return split_operand(filter, d->k, kk, kk, prepared + prepared_filter_floats(d->k, d->r, d->s, d->c), as_stream(stream));
+		}
 	}
 	return check_launch();
 }
@@ -443,10 +513,18 @@ int blob_convolution(void* stream, const nb200_conv_desc* d, const float* x, con
 		float* xs = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(scratch) + 15) & ~static_cast<uintptr_t>(15));
 		const float* fs = prepared;
 		const float* fprep = prepared != nullptr ? prepared + win.filterFloats : nullptr;
+		const bool split = precision == NB200_PREC_3XTF32 && split_form_pays(d, true);
+		const float* fsplit = prepared != nullptr ? prepared + 2 * win.filterFloats : nullptr;
 		pad_image_kernel<<<grid_for(static_cast<long long>(win.imageFloats / 4), 256, 16), 256, 0, as_stream(stream)>>>(
 			x, xs, d->batch, d->h, d->w, d->c, win.hp, win.wp, win.c4, d->pad_h, d->pad_w);
 		count_launch(1);
-		if(prepared == nullptr) {
+		if(prepared == nullptr && split) {
+			// (no larger than the two forms below, which the scratch has room for)
+			float* form = xs + (win.imageFloats + 3) / 4 * 4;
+			const int rc = split_window_filter(filter, d->k, d->r, d->s, d->c, win.c4, form, as_stream(stream));
+			if(rc != NB200_OK) return rc;
+			fsplit = form;
+		} else if(prepared == nullptr) {
 			float* widened = xs + (win.imageFloats + 3) / 4 * 4;
 			prepare_window_filter(stream, d, &win, filter, widened, precision);
 			fs = widened;
@@ -455,9 +533,10 @@ int blob_convolution(void* stream, const nb200_conv_desc* d, const float* x, con
 		int rc = check_launch();
 		if(rc != NB200_OK) return rc;
 		ContractionParams p = {};
-		p.A = xs; p.B = precision == NB200_PREC_3XTF32 ? fs : fprep; p.C = y;
-		p.Blo = precision == NB200_PREC_3XTF32 ? fprep : nullptr;
+		p.A = xs; p.B = split ? filter : precision == NB200_PREC_3XTF32 ? fs : fprep; p.C = y;
+		p.Blo = precision == NB200_PREC_3XTF32 && !split ? fprep : nullptr;
 		p.b_ready = 1;
+		if(split) set_split_operand(p, fsplit, d->k, d->r * 32LL);
 		p.M = d->batch * d->ho * d->wo; p.N = d->k; p.K = d->r * 32;
 		p.lda = 0; p.ldb = p.K; p.ldc = d->k;
 		p.a_mode = A_CONV_WINDOW; p.b_mode = B_ROWS; p.a_vec = 1; p.b_vec = 1;
@@ -539,8 +618,17 @@ int blob_convolution(void* stream, const nb200_conv_desc* d, const float* x, con
 		// costs more than converting those tiles in the kernel (ResNet-50 at batch 1: 0.69 -> 0.62 ms per pass)
 		const bool prepare = outRows >= PREPARE_B_MIN_ROWS;
 		if(prepare) {
-			const float* ready = prepared;
-			if(ready == nullptr || !aligned16(ready)) {
+			const bool given = prepared != nullptr && aligned16(prepared);
+			// the fp16 kernel's form where the launch is large enough; a caller whose room (a fixed array) is too small
+			// for its scales keeps the TF32 kernel
+			const bool split = precision == NB200_PREC_3XTF32 && split_form_pays(d, false)
+				&& (given || scratchFloats >= static_cast<size_t>(inScratch - scratch) + split_operand_floats(d->k, kk));
+			const float* ready = given ? prepared + (split ? prepared_filter_floats(d->k, d->r, d->s, d->c) : 0) : nullptr;
+			if(ready == nullptr && split) {
+				const int rc = split_operand(filter, d->k, kk, static_cast<int>(kk), inScratch, as_stream(stream));
+				if(rc != NB200_OK) return rc;
+				ready = inScratch;
+			} else if(ready == nullptr) {
 				const long long n = static_cast<long long>(d->k) * kk;
 				launch_dependent(overlap_launches(), prepare_filter_kernel, dim3(grid_for(n, 256, 8)), dim3(256), 0, as_stream(stream),
 					filter, inScratch, n, precision == NB200_PREC_3XTF32 ? 0 : 1);
@@ -549,7 +637,9 @@ int blob_convolution(void* stream, const nb200_conv_desc* d, const float* x, con
 				if(rc != NB200_OK) return rc;
 				ready = inScratch;
 			}
-			if(precision == NB200_PREC_3XTF32) p.Blo = ready; else p.B = ready;
+			if(split) set_split_operand(p, ready, d->k, kk);
+			else if(precision == NB200_PREC_3XTF32) p.Blo = ready;
+			else p.B = ready;
 			p.b_ready = 1;
 		}
 		// whatever the caller's scratch holds beyond the prepared filter is room for split-K partial results
@@ -565,6 +655,7 @@ int blob_convolution(void* stream, const nb200_conv_desc* d, const float* x, con
 		// the launcher could not describe an operand to TMA after all: fall back to in-kernel conversion
 		p.B = filter;
 		p.Blo = nullptr;
+		p.bSplit = nullptr;
 		p.b_ready = 0;
 		p.splitScratch = nullptr;
 	}

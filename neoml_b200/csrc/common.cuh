@@ -116,6 +116,18 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity)
 	return done != 0;
 }
 
+// One look at the barrier, without waiting; the lanes of a converged warp agree on the answer.
+__device__ __forceinline__ bool mbar_test_warp(uint64_t* bar, uint32_t parity)
+{
+	uint32_t done;
+	asm volatile(
+		"{\n\t.reg .pred P;\n\t"
+		"mbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+		"selp.b32 %0, 1, 0, P;\n\t}"
+		: "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+	return __all_sync(0xffffffffu, done != 0) != 0;
+}
+
 __device__ __forceinline__ uint64_t global_timer_ns()
 {
 	uint64_t t;
@@ -264,6 +276,17 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r)
 		  "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
 		: "memory");
 }
+__device__ __forceinline__ void tmem_ld8_issue(uint32_t taddr, uint32_t* r)
+{
+	asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+		: "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+		: "r"(taddr));
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r)
+{
+	asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+		::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
 __device__ __forceinline__ void tmem_st_wait()
 {
 	asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -271,6 +294,20 @@ __device__ __forceinline__ void tmem_st_wait()
 __device__ __forceinline__ void tmem_ld_wait()
 {
 	asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// -- register split -----------------------------------------------------------------------------------------------
+// Whole warpgroups (four warps) give up registers, or take what others of the block have given up.  To be called at the
+// head of the branch that only the warpgroup runs: the compiler allots registers from there on.
+template<int REGS>
+__device__ __forceinline__ void registers_down()
+{
+	asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS));
+}
+template<int REGS>
+__device__ __forceinline__ void registers_up()
+{
+	asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS));
 }
 
 // -- UMMA descriptors --------------------------------------------------------------------------------------------
@@ -320,6 +357,23 @@ __device__ __forceinline__ void umma_tf32_ts(uint32_t tmem_d, uint32_t tmem_a, u
 		"{\n\t.reg .pred p;\n\t"
 		"setp.ne.b32 p, %4, 0;\n\t"
 		"tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
+		::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+		: "memory");
+}
+
+// The same for fp16 operands (kind::f16, fp32 accumulate): 128 rows x 16 elements of K, two elements per column of tensor
+// memory (the even one in the low half); B rows hold 64 halves per 128 bytes.
+__host__ __device__ constexpr uint32_t umma_idesc_f16(int m, int n)
+{
+	return (1u << 4) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
+}
+__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
+	uint32_t accumulate)
+{
+	asm volatile(
+		"{\n\t.reg .pred p;\n\t"
+		"setp.ne.b32 p, %4, 0;\n\t"
+		"tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
 		::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
 		: "memory");
 }

@@ -34,6 +34,9 @@ struct ContractionParams {
 	int b_tma;  // B arrives by TMA (tiled rows)
 	const float* Blo; // optional: lo(B) = B - trunc_tf32(B) prepared by the caller (same shape and strides as B); with it,
 	                  // and for plain TF32 a pre-rounded B passed as B itself, the kernel does no per-step work on B
+	const float* bSplit; // optional (3xTF32, all-TMA first operand): B in the split form of split_operand(); the launch then goes
+	                     // to the fp16 kernel of contraction_split.cu
+	const float* bScale; // with bSplit: 1 / s_n of its rows, batch entries one after another
 	int kSplits;      // > 1: every tile's K loop is cut into this many equal parts that run as separate work items (few-tile
 	                  // launches: latency at small batch).  Part i stores its partial result at C + i * M * ldc, where C
 	                  // is then the caller's split scratch; a finishing pass sums the parts in order (deterministic) and
@@ -112,6 +115,18 @@ __device__ __forceinline__ float gather_b(const ContractionParams& p, const floa
 
 void set_contraction_trace(unsigned long long* buffer, int steps, int options);
 int launch_contraction_tc(const ContractionParams& p, int batch, cudaStream_t stream);
+int launch_contraction_split(const ContractionParams& p, int batch, cudaStream_t stream);
+int contraction_tile_width(int n);
+// Tensor maps (CUtensorMap behind the void pointer), contraction_tc.cu
+bool make_rows_map(void* map, const float* base, int k, long long rows, long long ld, int batch, long long batchStride, int boxRows);
+int make_operand_map(void* map, const ContractionParams& p, int batch, int boxRows);
+bool timing_events(cudaEvent_t* start, cudaEvent_t* stop);
+// The split form of a [rows x k] operand (rows `ld` floats apart, 16-byte aligned): floats it
+// takes, and the kernel that makes it; the row scales follow the rows at rows * (k rounded up to 32).
+size_t split_operand_floats(long long rows, long long k);
+int split_operand(const float* x, long long rows, long long ld, int k, float* out, cudaStream_t stream);
+// the same of a few-channel convolution's filter [rows][r][s][c], each filter row widened to 32 floats
+int split_window_filter(const float* f, int rows, int r, int s, int c, int c4, float* out, cudaStream_t stream);
 int launch_contraction_simt(const ContractionParams& p, int batch, cudaStream_t stream);
 
 // Event timing of the contraction launches (diagnostics.h)

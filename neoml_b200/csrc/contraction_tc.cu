@@ -904,8 +904,10 @@ void lookup_encoders()
 	});
 }
 
+} // namespace
+
 // Row-addressed operand as a 3-D tensor (k fastest, then rows, then batch); box = 32 k x boxRows rows, 128-byte swizzle.
-bool make_rows_map(CUtensorMap* map, const float* base, int k, long long rows, long long ld, int batch,
+bool make_rows_map(void* map, const float* base, int k, long long rows, long long ld, int batch,
 	long long batchStride, int boxRows)
 {
 	lookup_encoders();
@@ -917,10 +919,12 @@ bool make_rows_map(CUtensorMap* map, const float* base, int k, long long rows, l
 	if(strides[0] >= (1ull << 40) || strides[1] >= (1ull << 40)) return false;
 	const cuuint32_t box[3] = { BK, static_cast<cuuint32_t>(boxRows), 1 };
 	const cuuint32_t elemStrides[3] = { 1, 1, 1 };
-	return g_encodeTiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(base), dims, strides, box,
+	return g_encodeTiled(static_cast<CUtensorMap*>(map), CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(base), dims, strides, box,
 		elemStrides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
 		CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
+
+namespace {
 
 // Channels-last image (C, W, H, N) in im2col mode: a load delivers 128 consecutive output positions x 32 channels of
 // one filter tap; the window origins run over [-pad, dim + pad - (filter - 1) * dilation) with the convolution stride.
@@ -964,6 +968,15 @@ bool make_window_map(CUtensorMap* map, const ContractionParams& p, int images, i
 }
 
 } // namespace
+
+// The tensor map of the first operand: 1 = plain rows, 2 = im2col, 3 = row windows; 0 where TMA cannot describe it.
+int make_operand_map(void* map, const ContractionParams& p, int batch, int boxRows)
+{
+	CUtensorMap* m = static_cast<CUtensorMap*>(map);
+	if(p.a_mode == A_ROWS) return p.a_vec && make_rows_map(m, p.A, p.K, p.M, p.lda, batch, p.strideA, boxRows) ? 1 : 0;
+	if(p.a_mode == A_CONV_WINDOW) return batch == 1 && make_window_map(m, p, p.M / (p.Ho * p.Wo), p.K / BK) ? 3 : 0;
+	return p.a_vec && batch == 1 && make_im2col_map(m, p, p.M / (p.Ho * p.Wo), p.K / (p.S * p.Cin)) ? 2 : 0;
+}
 
 // Channels-last image batch (C, W, H, N) as a plain tiled map without swizzle: a load delivers a box of boxC channels x
 // boxW columns x boxH rows of one image, zeros where the box leaves the image (a convolution's padding for free).
@@ -1042,6 +1055,8 @@ struct LaunchTiming {
 LaunchTiming g_timing;
 thread_local double t_callFlops = 0.0;
 
+} // namespace
+
 // the next pair of events (created on first use, reused afterwards); false when timing is off
 bool timing_events(cudaEvent_t* start, cudaEvent_t* stop)
 {
@@ -1062,6 +1077,8 @@ bool timing_events(cudaEvent_t* start, cudaEvent_t* stop)
 	++g_timing.used;
 	return true;
 }
+
+namespace {
 
 unsigned long long* g_traceBuffer = nullptr;
 int g_traceSteps = 0;
@@ -1119,15 +1136,7 @@ int launch_bn(const ContractionParams& p0, int batch, cudaStream_t stream)
 	p.a_tma = 0;
 	p.b_tma = 0;
 	if(!(g_traceOptions & 16)) {
-		if(p.a_mode == A_ROWS) {
-			if(p.a_vec && make_rows_map(&mapA, p.A, p.K, p.M, p.lda, batch, p.strideA, BM)) p.a_tma = 1;
-		} else if(p.a_mode == A_CONV_WINDOW) {
-			if(batch == 1 && make_window_map(&mapA, p, p.M / (p.Ho * p.Wo), p.K / BK)) p.a_tma = 3;
-		} else if(p.a_vec && batch == 1) {
-			const int filterH = p.K / (p.S * p.Cin);
-			const int images = p.M / (p.Ho * p.Wo);
-			if(make_im2col_map(&mapA, p, images, filterH)) p.a_tma = 2;
-		}
+		p.a_tma = make_operand_map(&mapA, p, batch, BM);
 		if(p.b_mode == B_ROWS && p.b_vec && make_rows_map(&mapB, p.B, p.K, p.N, p.ldb, batch, p.strideB, BN)) p.b_tma = 1;
 	}
 	if(p.a_mode == A_CONV_WINDOW && (p.a_tma != 3 || !p.b_tma)) return NB200_EINVAL; // no gather form of this mode
@@ -1264,19 +1273,25 @@ void set_contraction_trace(unsigned long long* buffer, int steps, int options)
 	g_traceOptions = options;
 }
 
-int launch_contraction_tc(const ContractionParams& p, int batch, cudaStream_t stream)
+// tile width: least zero-padded columns over all tiles; ties go to the wider tile (fewer re-reads of A)
+int contraction_tile_width(int n)
 {
-	if(p.M <= 0 || p.N <= 0 || batch <= 0) return NB200_OK;
-	if(p.K <= 0) return NB200_EINVAL;
-	// tile width: least zero-padded columns over all tiles; ties go to the wider tile (fewer re-reads of A)
 	const int widths[4] = { 128, 96, 64, 32 };
 	int best = 128;
 	long long bestPadded = -1;
 	for(int i = 0; i < 4; ++i) {
-		const long long padded = (static_cast<long long>(p.N) + widths[i] - 1) / widths[i] * widths[i];
+		const long long padded = (static_cast<long long>(n) + widths[i] - 1) / widths[i] * widths[i];
 		if(bestPadded < 0 || padded < bestPadded) { bestPadded = padded; best = widths[i]; }
 	}
-	switch(best) {
+	return best;
+}
+
+int launch_contraction_tc(const ContractionParams& p, int batch, cudaStream_t stream)
+{
+	if(p.M <= 0 || p.N <= 0 || batch <= 0) return NB200_OK;
+	if(p.K <= 0) return NB200_EINVAL;
+	if(p.bSplit != nullptr) return (g_traceOptions & 16) ? NB200_EINVAL : launch_contraction_split(p, batch, stream);
+	switch(contraction_tile_width(p.N)) {
 		case 32: return launch_bn<32>(p, batch, stream);
 		case 64: return launch_bn<64>(p, batch, stream);
 		case 96: return launch_bn<96>(p, batch, stream);

@@ -1,0 +1,96 @@
+"""The fp16 contraction kernel (neoml_b200/csrc/contraction_split.cu) at the edges of its tiles and of its number range.
+
+Bound of the comparison, against sums in double precision and relative to sum |a||b| of each result: three split errors of
+at most 2^-22, and one truncation of at most 2^-22 for each of the ceil(K / 16) accumulations (main and cross) and for the
+epilogue's four roundings."""
+from __future__ import annotations
+
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from neoml_b200 import ops as module
+    return module
+
+
+def bound(k: int) -> float:
+    return (3 + math.ceil(k / 16) + 4) * 2.0 ** -22
+
+
+def worst(got, a, b, extra=None):
+    want = a.double() @ b.double().transpose(-1, -2)
+    size = a.abs().double() @ b.abs().double().transpose(-1, -2)
+    if extra is not None:
+        want, size = want + extra.double(), size + extra.abs().double()
+    assert bool((got[size == 0] == 0).all())
+    return float(((got.double() - want).abs() / size.clamp_min(1e-300)).max())
+
+
+def rows_of(kind: str, m: int, k: int, g) -> torch.Tensor:
+    a = torch.empty(m, k, device="cuda").normal_(generator=g)
+    if kind == "zeros":          # rows without anything, rows that begin with empty K blocks, a ReLU's half
+        a.clamp_(min=0)
+        a[::2, : k // 2] = 0
+        a[::5] = 0
+    elif kind == "scales":       # every row of another magnitude, over fp32's range
+        a *= torch.logspace(-30, 30, m, device="cuda")[:, None]
+    elif kind == "rising":       # every K block beyond the range of the one before: the row scales move in mid-tile
+        a *= torch.pow(2.0, 7.0 * (torch.arange(k, device="cuda") // 32).clamp(max=12))
+    elif kind == "jump":         # some rows of a warp move, others do not; the last block included
+        a[::3, k // 2:] *= 1e4
+        a[1::7, k - 1] *= 1e6
+    return a
+
+
+# m x k x n: 75 row tiles are the fewest that one column tile takes to this kernel, 160 = five K blocks the shortest depth
+@pytest.mark.parametrize("m,k,n", [(75 * 128 - 127, 160, 32), (9700, 132, 57), (9600, 190, 64), (9601, 576, 96), (4800, 320, 129),
+                                   (1024, 333 * 4, 1300), (5000, 2064, 260)])
+@pytest.mark.parametrize("kind", ["normal", "zeros", "scales", "rising", "jump"])
+def test_products(ops, m, k, n, kind):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(m + k)
+    a, b = rows_of(kind, m, k, g), torch.empty(n, k, device="cuda").normal_(generator=g)
+    b *= torch.logspace(-3, 3, n, device="cuda")[:, None]
+    got = ops.MultiplyMatrixByTransposedMatrix(a, b)
+    assert worst(got, a, b) < bound(k)
+    assert torch.equal(got, ops.MultiplyMatrixByTransposedMatrix(a, b))
+    if kind in ("normal", "jump"):
+        bias, res = torch.empty(n, device="cuda").normal_(generator=g), torch.empty(m, n, device="cuda").normal_(generator=g)
+        got = ops.MultiplyMatrixByTransposedMatrix(a, b, free_term=bias, residual=res)
+        assert worst(got, a, b, extra=bias + res) < bound(k)
+
+
+def test_batches_and_infinities(ops):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    a = torch.empty(7, 1100, 160, device="cuda").normal_(generator=g)
+    b = torch.empty(7, 200, 160, device="cuda").normal_(generator=g)
+    assert worst(ops.BatchMultiplyMatrixByTransposedMatrix(a, b), a, b) < bound(160)
+    a[2, 5, 3], a[2, 7, 159] = float("inf"), float("nan")
+    got = ops.BatchMultiplyMatrixByTransposedMatrix(a, b)
+    assert not bool(torch.isfinite(got[2, 5]).any()) and bool(torch.isnan(got[2, 7]).all())
+    a[2, 5, 3] = a[2, 7, 159] = 0.0
+    rest = ops.BatchMultiplyMatrixByTransposedMatrix(a, b)
+    keep = torch.ones(7, 1100, dtype=torch.bool, device="cuda")
+    keep[2, 5] = keep[2, 7] = False
+    assert torch.equal(got[keep], rest[keep])      # the other rows of the tile do not notice
+
+
+@pytest.mark.parametrize("shape,k,r,stride,pad,dil", [((5, 45, 47, 64), 70, 3, 1, 1, 1), ((3, 61, 59, 32), 128, 5, 2, 2, 1),
+                                                      ((9, 31, 33, 32), 96, 3, 1, 2, 2), ((4, 75, 90, 3), 64, 7, 2, 3, 1)])
+def test_convolutions(ops, shape, k, r, stride, pad, dil):
+    """im2col and row-window operands; the padding's zeros come first in the border rows."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(k)
+    x, f = torch.empty(shape, device="cuda").normal_(generator=g), torch.empty(k, r, r, shape[3], device="cuda").normal_(generator=g)
+    got = ops.BlobConvolution(x, f, padding=(pad, pad), stride=(stride, stride), dilation=(dil, dil))
+    conv = lambda p, q: torch.nn.functional.conv2d(p.double().permute(0, 3, 1, 2), q.double().permute(0, 3, 1, 2), stride=stride,
+                                                   padding=pad, dilation=dil).permute(0, 2, 3, 1)
+    err = (got.double() - conv(x, f)).abs() / conv(x.abs(), f.abs()).clamp_min(1e-300)
+    assert float(err.max()) < bound(r * r * shape[3])
