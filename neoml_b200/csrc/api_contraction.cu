@@ -85,6 +85,34 @@ __global__ void __launch_bounds__(256) prepare_filter_kernel(const float* __rest
 	}
 }
 
+// The operands of a product whose rows are not whole 16-byte pieces (an odd depth), copied into rows that are: y[r][0..k) of
+// rows k4 floats apart = x[r][0..k) of rows ld apart; the floats between k and k4 are never read.  A warp per row, both
+// operands in one launch.  Bound: memory (4-byte accesses, each row coalesced).  It buys the TMA-fed kernels: their
+// cp.async twin fetches such rows float by float, 5.9 us per K block of 128 x 96 tiles whatever their number below a wave.
+// Both operands copied and multiplied against gathered: 5 x (333 x 517 x 259) 25.7 us against 99.9, 2000 x 1003 x 1005 47.6
+// against 218, 16 x 17 x 33 8.0 against 12.2, 90 x (100 x 33 x 65) 16.2 against 28.2: no size was found where it loses.
+struct RepackRows {
+	const float* x;
+	float* y;
+	long long rows, ld;
+};
+__global__ void __launch_bounds__(256) repack_rows_kernel(const RepackRows first, const RepackRows second, int k, int k4)
+{
+	// the scratch this writes may still be read by the product before it in the stream
+	dependent_wait();
+	dependents_may_start();
+	const int lane = threadIdx.x & 31;
+	const long long warps = static_cast<long long>(gridDim.x) * 8;
+	for(long long r = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5); r < first.rows + second.rows; r += warps) {
+		const bool inFirst = r < first.rows;
+		const long long row = inFirst ? r : r - first.rows;
+		const float* src = inFirst ? first.x + row * first.ld : second.x + row * second.ld;
+		float* dst = (inFirst ? first.y : second.y) + row * k4;
+#pragma unroll 8
+		for(int i = lane; i < k; i += 32) dst[i] = __ldg(src + i);
+	}
+}
+
 // Room for the partial results of a split-K launch: only launches with few tiles split (at most 74 tiles of 128 x 128
 // outputs, cut in as many parts as fill the machine), so the product of parts and outputs is bounded.
 constexpr long long SPLIT_TILES_MAX = 74;
@@ -305,9 +333,20 @@ int nb200_batch_multiply_matrix_by_transposed_matrix(void* stream, int batch, co
 	return run(p, batch, stream, precision);
 }
 
-size_t nb200_matrix_product_scratch_floats(int batch, int m, int n, int k, int ldb)
+// Products whose scratch has room for both operands in 16-byte rows
+static bool repack_wanted(int k, int ldb)
 {
-	if(batch <= 0 || m <= 0 || n <= 0 || k <= 0 || ldb < k) return 0;
+	return k % 4 != 0 || ldb % 4 != 0;
+}
+
+static size_t repack_floats(int batch, int m, int n, int k)
+{
+	return static_cast<size_t>(batch) * (static_cast<size_t>(m) + n) * ((k + 3) / 4 * 4) + 8;
+}
+
+// ... for a product whose rows are whole 16-byte pieces
+static size_t aligned_product_floats(int batch, int m, int n, int k, int ldb)
+{
 	size_t floats = 0;
 	// the split second operand pays when it is reused by several row tiles
 	if(m >= PREPARE_B_MIN_ROWS) {
@@ -322,10 +361,21 @@ size_t nb200_matrix_product_scratch_floats(int batch, int m, int n, int k, int l
 	return floats;
 }
 
+size_t nb200_matrix_product_scratch_floats(int batch, int m, int n, int k, int ldb)
+{
+	if(batch <= 0 || m <= 0 || n <= 0 || k <= 0 || ldb < k) return 0;
+	if(!repack_wanted(k, ldb)) return aligned_product_floats(batch, m, n, k, ldb);
+	// room for the rows as they are, or for the copies and what their product wants (depths that are no multiple of four
+	// in rows that are aligned all the same need no copies)
+	const size_t as_is = aligned_product_floats(batch, m, n, k, ldb);
+	const size_t copied = repack_floats(batch, m, n, k) + aligned_product_floats(batch, m, n, k, (k + 3) / 4 * 4);
+	return as_is > copied ? as_is : copied;
+}
+
 // The product behind the three entry points below.  `prepared` (optional, batch 1): the second operand in the form
 // nb200_matrix_product_prepare_second makes, kept by the caller for as long as the operand does not change.
 static int matrix_product(void* stream, int batch, const float* a, int m, int k, int lda, const float* b, int n, int ldb,
-	float* c, int ldc, float* scratch, const float* prepared, const nb200_epilogue* epi, int precision)
+	float* c, int ldc, float* scratch, const float* prepared, const nb200_epilogue* epi, int precision, bool repacked = false)
 {
 	if(batch < 0 || m < 0 || n < 0 || k <= 0 || lda < k || ldb < k || ldc < n) return NB200_EINVAL;
 	set_call_flops(2.0 * batch * m * n * k);
@@ -339,6 +389,23 @@ static int matrix_product(void* stream, int batch, const float* a, int m, int k,
 	fill_epilogue(p, epi);
 	if(p.residual == nullptr) p.ldr = ldc;
 	p.a_vec = vec_ok(a, lda, p.strideA); p.b_vec = vec_ok(b, ldb, p.strideB);
+	p.separate_cross = repacked ? 1 : 0; // short depths: the bits of the kernel that gathers the rows as they are
+	if(scratch != nullptr && repack_wanted(k, ldb) && (!p.a_vec || !p.b_vec) && a != nullptr && b != nullptr && batch > 0 && m > 0 && n > 0
+		&& (precision == NB200_PREC_3XTF32 || precision == NB200_PREC_TF32) && !gather_forced()
+		&& static_cast<long long>(m) * ((k + 3) / 4 * 4) <= 0x7fffffffLL && static_cast<long long>(m) * ldc <= 0x7fffffffLL) {
+		if(device_status_word() == nullptr) return NB200_ENODEVICE;
+		const int k4 = (k + 3) / 4 * 4;
+		float* rowsA = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(scratch) + 15) & ~static_cast<uintptr_t>(15));
+		const RepackRows first = { a, rowsA, static_cast<long long>(batch) * m, lda };
+		const RepackRows second = { b, rowsA + first.rows * k4, static_cast<long long>(batch) * n, ldb };
+		launch_dependent(overlap_launches(), repack_rows_kernel, dim3(grid_for(first.rows + second.rows, 8, 8)), dim3(256), 0,
+			as_stream(stream), first, second, k, k4);
+		count_launch(1);
+		const int rc = check_launch();
+		if(rc != NB200_OK) return rc;
+		return matrix_product(stream, batch, rowsA, m, k, k4, second.y, n, k4, c, ldc,
+			aligned_product_floats(batch, m, n, k, k4) > 0 ? second.y + second.rows * k4 : nullptr, nullptr, epi, precision, true);
+	}
 	const bool plain = precision == NB200_PREC_FP32_SIMT || batch == 0 || m == 0 || n == 0 || !p.a_vec || !p.b_vec
 		|| static_cast<long long>(batch) * n * ldb > 0x7fffffffLL;
 	if(plain || (scratch == nullptr && prepared == nullptr)) return run(p, batch, stream, precision);

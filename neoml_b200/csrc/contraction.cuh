@@ -41,6 +41,7 @@ struct ContractionParams {
 	                  // launches: latency at small batch).  Part i stores its partial result at C + i * M * ldc, where C
 	                  // is then the caller's split scratch; a finishing pass sums the parts in order (deterministic) and
 	                  // applies bias, residual and activation.  Set by the launcher.
+	int separate_cross; // 1: no short-K variant (which adds the cross products into the main accumulator)
 	int b_resident;   // set by the launcher (short-K kernels): B stays in shared memory for all tiles of a CTA
 	float* splitScratch;          // optional room for those partial results (NULL: never split)
 	long long splitScratchFloats;

@@ -1178,7 +1178,7 @@ int launch_bn(const ContractionParams& p0, int batch, cudaStream_t stream)
 	// (-7 %) and loses from eight on.
 	bool shortK = false;
 	p.b_resident = 0;
-	if(!gather && kSplits == 1 && numKb <= 4 && p.a_mode != A_CONV_WINDOW && !(g_traceOptions & 128)) {
+	if(!gather && kSplits == 1 && numKb <= 4 && p.a_mode != A_CONV_WINDOW && p.separate_cross == 0 && !(g_traceOptions & 128)) {
 		const int resRing = p.residual != nullptr && p.c_vec ? MAX_EPI_WARPS * RES_DEPTH * STAGING_BYTES_PER_WARP : 0;
 		const int residentBytes = numKb * bStepBytes;
 		const int room = 227 * 1024 - fixedBytes - resRing - residentBytes;

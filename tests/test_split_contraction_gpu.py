@@ -94,3 +94,24 @@ def test_convolutions(ops, shape, k, r, stride, pad, dil):
                                                    padding=pad, dilation=dil).permute(0, 2, 3, 1)
     err = (got.double() - conv(x, f)).abs() / conv(x.abs(), f.abs()).clamp_min(1e-300)
     assert float(err.max()) < bound(r * r * shape[3])
+
+
+# rows of 4k + 1..3 floats: both operands are copied into 16-byte rows first.  Where the product then runs on the TF32
+# kernel unsplit it forms the same sums in the same order as the kernel that gathers the rows as they are
+@pytest.mark.parametrize("batch,m,k,n,same", [(1, 1, 5, 1, True), (3, 40, 33, 50, True), (2, 129, 127, 97, True), (90, 65, 61, 33, True),
+                                              (1, 200, 1001, 131, False), (1, 2000, 1003, 905, False), (2, 5000, 131, 70, False)])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_odd_depths(ops, batch, m, k, n, same, precision):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(k)
+    a, b = torch.empty(batch, m, k, device="cuda").normal_(generator=g), torch.empty(batch, n, k, device="cuda").normal_(generator=g)
+    got = ops.BatchMultiplyMatrixByTransposedMatrix(a, b, precision=precision)
+    gathered = ops.BatchMultiplyMatrixByTransposedMatrix(a, b, precision=precision, use_scratch=False)
+    if same:
+        assert torch.equal(got, gathered)
+    # TF32 operands are rounded to 11 bits: two errors of 2^-12 more; the TF32 kernel accumulates 8 products at a time
+    limit = 2 * bound(k) + (2.0 ** -11 if precision else 0.0)
+    assert worst(got, a, b) < limit
+    odd = torch.nn.functional.pad(a[0], (0, 2)).contiguous()     # an odd row length in memory, too
+    wide = ops.MultiplyMatrixByTransposedMatrix(odd, b[0], first_width=k, precision=precision, first_row_size=k + 2)
+    assert worst(wide, a[0], b[0]) < limit
