@@ -418,6 +418,7 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 		int stripCol = -1, stripBatch = -1;
 		const bool fastStore = vec && p.accumulate == 0 && p.act != NB200_ACT_HSWISH && p.act != NB200_ACT_SIGMOID_GATE;
 		const bool gateStore = vec && p.accumulate == 0 && p.act == NB200_ACT_SIGMOID_GATE;
+		const bool hswishStore = vec && p.accumulate == 0 && p.act == NB200_ACT_HSWISH;
 		const bool clampOn = p.act == NB200_ACT_RELU;
 		const float actParam = p.act_param_device != nullptr ? __ldg(p.act_param_device) : p.act_param;
 		const float clampHi = actParam > 0.f ? actParam : __int_as_float(0x7f800000);
@@ -564,6 +565,20 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 						if(useRes) { o.x += res[i].x; o.y += res[i].y; o.z += res[i].z; o.w += res[i].w; }
 						o.x = apply_act(o.x, NB200_ACT_SIGMOID_GATE, actParam); o.y = apply_act(o.y, NB200_ACT_SIGMOID_GATE, actParam);
 						o.z = apply_act(o.z, NB200_ACT_SIGMOID_GATE, actParam); o.w = apply_act(o.w, NB200_ACT_SIGMOID_GATE, actParam);
+						float* dst = C + static_cast<size_t>(m) * p.ldc + n;
+						if(m < mEnd) {
+							asm volatile("st.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(o.x), "f"(o.y), "f"(o.z), "f"(o.w) : "memory");
+						}
+					}
+				} else if(hswishStore && colsFull) {
+					// and with the hard swish (the element-wise path below takes twice as long: an expand layer of 24 -> 144 channels)
+#pragma unroll
+					for(int i = 0; i < 4; ++i) {
+						const int m = rowBase + 8 * i + rowInGroup;
+						float4 o = ov[i];
+						if(useRes) { o.x += res[i].x; o.y += res[i].y; o.z += res[i].z; o.w += res[i].w; }
+						o.x = apply_act(o.x, NB200_ACT_HSWISH, actParam); o.y = apply_act(o.y, NB200_ACT_HSWISH, actParam);
+						o.z = apply_act(o.z, NB200_ACT_HSWISH, actParam); o.w = apply_act(o.w, NB200_ACT_HSWISH, actParam);
 						float* dst = C + static_cast<size_t>(m) * p.ldc + n;
 						if(m < mEnd) {
 							asm volatile("st.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(o.x), "f"(o.y), "f"(o.z), "f"(o.w) : "memory");
@@ -773,7 +788,8 @@ int split_window_filter(const float* f, int rows, int r, int s, int c, int c4, f
 int launch_contraction_split(const ContractionParams& p, int batch, cudaStream_t stream)
 {
 	if(p.M <= 0 || p.N <= 0 || batch <= 0) return NB200_OK;
-	switch(contraction_tile_width(p.N)) {
+	const int tileM = p.a_mode == A_CONV_WINDOW && p.tileM > 0 && p.tileM <= BM ? p.tileM : BM;
+	switch(balanced_tile_width((p.M + tileM - 1LL) / tileM, p.N, batch)) {
 		case 32: return launch_bn<32>(p, batch, stream);
 		case 64: return launch_bn<64>(p, batch, stream);
 		case 96: return launch_bn<96>(p, batch, stream);

@@ -631,6 +631,7 @@ __global__ void __maxnreg__(128) contraction_tc_kernel(const ContractionParams p
 		// uniform epilogue options, decided once: the fast store path has no branch per element
 		const bool fastStore = vec && p.accumulate == 0 && p.act != NB200_ACT_HSWISH && p.act != NB200_ACT_SIGMOID_GATE;
 		const bool gateStore = vec && p.accumulate == 0 && p.act == NB200_ACT_SIGMOID_GATE;
+		const bool hswishStore = vec && p.accumulate == 0 && p.act == NB200_ACT_HSWISH;
 		const bool clampOn = p.act == NB200_ACT_RELU;
 		const float actParam = p.act_param_device != nullptr ? __ldg(p.act_param_device) : p.act_param;
 		const float clampHi = actParam > 0.f ? actParam : __int_as_float(0x7f800000);
@@ -821,6 +822,21 @@ __global__ void __maxnreg__(128) contraction_tc_kernel(const ContractionParams p
 							if(useRes) { o.x += res[i].x; o.y += res[i].y; o.z += res[i].z; o.w += res[i].w; }
 							o.x = apply_act(o.x, NB200_ACT_SIGMOID_GATE, actParam); o.y = apply_act(o.y, NB200_ACT_SIGMOID_GATE, actParam);
 							o.z = apply_act(o.z, NB200_ACT_SIGMOID_GATE, actParam); o.w = apply_act(o.w, NB200_ACT_SIGMOID_GATE, actParam);
+							float* dst = C + static_cast<size_t>(m) * p.ldc + n;
+							if(m < mEnd) {
+								asm volatile("st.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(o.x), "f"(o.y), "f"(o.z), "f"(o.w) : "memory");
+							}
+						}
+					} else if(hswishStore && colsFull) {
+						// and with the hard swish (the element-wise path below takes twice as long: an expand layer of 24 -> 144 channels)
+#pragma unroll
+						for(int i = 0; i < 4; ++i) {
+							const int m = rowBase + 8 * i + rowInGroup;
+							float4 o = ov[i];
+							o.x += bias4.x; o.y += bias4.y; o.z += bias4.z; o.w += bias4.w;
+							if(useRes) { o.x += res[i].x; o.y += res[i].y; o.z += res[i].z; o.w += res[i].w; }
+							o.x = apply_act(o.x, NB200_ACT_HSWISH, actParam); o.y = apply_act(o.y, NB200_ACT_HSWISH, actParam);
+							o.z = apply_act(o.z, NB200_ACT_HSWISH, actParam); o.w = apply_act(o.w, NB200_ACT_HSWISH, actParam);
 							float* dst = C + static_cast<size_t>(m) * p.ldc + n;
 							if(m < mEnd) {
 								asm volatile("st.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(o.x), "f"(o.y), "f"(o.z), "f"(o.w) : "memory");
@@ -1286,12 +1302,35 @@ int contraction_tile_width(int n)
 	return best;
 }
 
+// The same where K is not split: the width whose waves over the SMs cost least.  A tile's K block is bound by the copies and
+// the conversion of A far more than by its columns: 128, 96, 64 and 32 of them measured 100 : 90 : 80 : 62 per wave with
+// either kernel (2048 x 1024 x 1300: 56, 51, 63, 86 us in 2, 2, 3, 5 waves).  The least-padded width made such a product
+// 32 columns wide: 1300 columns 86 us for 51, 20000 x 512 x 384 has 4 waves of 128 at 37 us against 13 of 32 at 81,
+// 100000 x 24 x 144 31 us for 25.
+int balanced_tile_width(long long mTiles, int n, int batch)
+{
+	const int widths[4] = { 128, 96, 64, 32 };
+	const long long cost[4] = { 100, 90, 80, 62 };
+	const int sms = sm_count();
+	int best = 128;
+	long long least = -1;
+	for(int i = 0; i < 4; ++i) {
+		const long long tiles = mTiles * ((n + widths[i] - 1) / widths[i]) * batch;
+		const long long total = (tiles + sms - 1) / sms * cost[i];
+		if(least < 0 || total < least) { least = total; best = widths[i]; }
+	}
+	return best;
+}
+
 int launch_contraction_tc(const ContractionParams& p, int batch, cudaStream_t stream)
 {
 	if(p.M <= 0 || p.N <= 0 || batch <= 0) return NB200_OK;
 	if(p.K <= 0) return NB200_EINVAL;
 	if(p.bSplit != nullptr) return (g_traceOptions & 16) ? NB200_EINVAL : launch_contraction_split(p, batch, stream);
-	switch(contraction_tile_width(p.N)) {
+	// (with room for split K, a few-tile launch keeps the least-padded width: its parts fill the machine whatever the width)
+	const bool maySplit = p.splitScratch != nullptr && batch == 1 && p.K >= 8 * BK;
+	const long long mTiles = (p.M + BM - 1LL) / BM;
+	switch(maySplit ? contraction_tile_width(p.N) : balanced_tile_width(mTiles, p.N, batch)) {
 		case 32: return launch_bn<32>(p, batch, stream);
 		case 64: return launch_bn<64>(p, batch, stream);
 		case 96: return launch_bn<96>(p, batch, stream);
