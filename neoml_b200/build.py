@@ -1,6 +1,7 @@
 """Builds the native parts of the package in-tree.
 
   neoml_b200/lib/libneoml_b200.so      CUDA kernels + C ABI (include/neoml_b200.h), sm_100a only
+  neoml_b200/lib/_ops_native.so        the native half of neoml_b200/ops.py
   neoml_b200/lib/libNeoMathEngineB200.so  C++ IMathEngine implementation over that C ABI; compiled against the
                                        NeoMathEngine headers of a NeoML checkout ($NEOML_REFERENCE_DIR), so it is
                                        only (re)built where such a checkout exists
@@ -120,9 +121,31 @@ def build_engine(verbose: bool = False) -> Path | None:
     return out
 
 
+def build_bindings(verbose: bool = False) -> Path:
+    """g++ build of the native half of neoml_b200/ops.py (a CPython module over torch's headers and the C ABI)."""
+    import sysconfig
+    import torch
+    src, out = ROOT / "bindings" / "ops_native.cpp", LIB / "_ops_native.so"
+    if not _newer(src, out, sorted(INCLUDE.glob("*.h"))):
+        return out
+    base = Path(torch.__file__).resolve().parent
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-w",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f"-I{base}/include",
+           f"-I{base}/include/torch/csrc/api/include", f"-I{sysconfig.get_paths()['include']}", "-I/usr/local/cuda/include",
+           str(src), "-o", str(out), f"-L{base}/lib", f"-L{LIB}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python",
+           "-lneoml_b200", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if verbose:
+        print(r.stdout + r.stderr)
+    if r.returncode != 0:
+        raise RuntimeError(f"bindings build failed:\n{r.stdout}{r.stderr}")
+    return out
+
+
 def main() -> None:
     verbose = "-v" in sys.argv
     print(build_kernels(verbose))
+    print(build_bindings(verbose))
     print(build_engine(verbose))
     print(build_hosted(verbose))
 

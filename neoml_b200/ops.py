@@ -8,11 +8,37 @@ channels-last ``[batch, height, width, channels]`` fp32 tensors, filters ``[coun
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 
 import torch
 
 from . import _capi as capi
 from ._capi import (ACT_HSWISH, ACT_NONE, ACT_RELU, PREC_3XTF32, PREC_FP32_SIMT, PREC_TF32, VEC)  # noqa: F401
+
+
+_native_module = None
+
+
+def _native():
+    """The native half of the calls below (bindings/ops_native.cpp): it answers None for arguments that it does not take,
+    and the Python code after the call then raises or handles them."""
+    global _native_module
+    if _native_module is None:
+        path = capi.LIB_PATH.parent / "_ops_native.so"
+        if not path.exists():
+            raise RuntimeError(f"{path} is missing: run `python -m neoml_b200.build` (no fallback exists)")
+        loader = importlib.machinery.ExtensionFileLoader("_ops_native", str(path))
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_ops_native", loader))
+        loader.exec_module(module)
+        _native_module = module
+    return _native_module
+
+
+def _checked(name: str, answer):
+    if type(answer) is int:
+        capi.check(name, answer)
+    return answer
 
 
 def _stream() -> int:
@@ -56,6 +82,10 @@ def MultiplyMatrixByTransposedMatrix(first, second, result=None, *, first_row_si
     lda = first_row_size if first_row_size is not None else k
     ldb = second_row_size if second_row_size is not None else k
     ldc = result_row_size if result_row_size is not None else n
+    done = _native().multiply_by_transposed(first, second, result, m, k, n, lda, ldb, ldc, free_term, residual, act, act_param,
+                                            accumulate, precision, use_scratch)
+    if done is not None:
+        return _checked("MultiplyMatrixByTransposedMatrix", done)
     if result is None:
         result = torch.empty((m, ldc), dtype=torch.float32, device=first.device)
     epi = _epilogue(free_term, residual, ldc, act, act_param, accumulate)
@@ -74,6 +104,9 @@ def MultiplyMatrixByTransposedMatrix(first, second, result=None, *, first_row_si
 
 def BatchMultiplyMatrixByTransposedMatrix(first, second, result=None, *, precision=PREC_3XTF32, use_scratch=True):
     """first [B, M, K], second [B, N, K] -> result [B, M, N]."""
+    done = _native().batch_multiply_by_transposed(first, second, result, precision, use_scratch)
+    if done is not None:
+        return _checked("BatchMultiplyMatrixByTransposedMatrix", done)
     b, m, k = first.shape
     n = second.shape[1]
     if result is None:
@@ -102,6 +135,10 @@ def MultiplyMatrixByMatrix(first, second, result=None, *, precision=PREC_3XTF32,
     squeeze = first.dim() == 2
     if squeeze:
         first, second = first.unsqueeze(0), second.unsqueeze(0)
+    done = _native().multiply_by_matrix(first, second, result, precision) if use_scratch else None
+    if done is not None:
+        done = _checked("MultiplyMatrixByMatrix", done)
+        return done[0] if squeeze else done
     b, m, k = first.shape
     n = second.shape[2]
     if result is None:
@@ -120,6 +157,10 @@ def MultiplyMatrixByMatrix(first, second, result=None, *, precision=PREC_3XTF32,
 
 def BlobConvolution(source, filter, free_term=None, result=None, *, padding=(0, 0), stride=(1, 1), dilation=(1, 1),
                     residual=None, act=ACT_NONE, act_param=0.0, precision=PREC_3XTF32, use_scratch=True):
+    done = _native().blob_convolution(source, filter, free_term, result, padding[0], padding[1], stride[0], stride[1],
+                                      dilation[0], dilation[1], residual, act, act_param, precision, use_scratch)
+    if done is not None:
+        return _checked("BlobConvolution", done)
     n, h, w, c = source.shape
     k, r, s, c2 = filter.shape
     assert c == c2
@@ -182,6 +223,9 @@ def MobileNetV2Block(source, expand_filter, expand_free_term, channelwise_filter
 def vector_op(op: str, first=None, second=None, scalar=None, value=0.0, result=None, count=None):
     """Elementwise family; `op` is one of capi.VEC_OPS.  `scalar` is a 1-element device tensor where the reference
     takes a handle (VectorMultiply, VectorReLU threshold, ...)."""
+    done = _native().vector_op(VEC[op], first, second, scalar, value, result, count)
+    if done is not None:
+        return _checked("Vector" + op, done)
     ref = first if first is not None else result
     if result is None:
         result = torch.empty_like(ref)
@@ -268,6 +312,9 @@ def MatrixSoftmaxByRowsFused(matrix, height, width, scale=None, row_bias=None, b
 
 
 def TransposeMatrix(batch, first, height, medium, width, channels, result=None):
+    done = _native().transpose(batch, first, height, medium, width, channels, result)
+    if done is not None:
+        return _checked("TransposeMatrix", done)
     if result is None:
         result = torch.empty_like(first)
     capi.check("TransposeMatrix", capi.load().nb200_transpose_matrix(

@@ -1,0 +1,35 @@
+"""The native half of neoml_b200/ops.py declines what it does not take, so that the Python code raises as it always did."""
+import pytest
+import torch
+
+from neoml_b200 import ops
+
+
+def test_native_calls_decline_other_tensors():
+    native = ops._native()
+    a, f = torch.zeros(2, 3, 4), torch.zeros(1, 3, 3, 4)
+    assert native.batch_multiply_by_transposed(a, a, None, 0, True) is None                  # not on a GPU
+    assert native.multiply_by_matrix(a, a, None, 0) is None
+    assert native.transpose(1, a, 2, 1, 3, 4, None) is None
+    assert native.vector_op(0, a, None, None, 0.0, None, None) is None
+    assert native.vector_op(0, None, None, None, 0.0, None, None) is None
+    assert native.blob_convolution(torch.zeros(1, 5, 5, 4), f, None, None, 0, 0, 1, 1, 1, 1, None, 0, 0.0, 0, True) is None
+    with pytest.raises(TypeError):
+        native.transpose(1, a)
+
+
+@pytest.mark.gpu
+def test_errors_are_the_python_codes():
+    x, f = torch.zeros(1, 5, 5, 4, device="cuda"), torch.zeros(2, 3, 3, 4, device="cuda")
+    y = ops.BlobConvolution(x, f)
+    assert y.shape == (1, 3, 3, 2) and y.device == x.device and y.dtype == torch.float32
+    with pytest.raises(AssertionError):
+        ops.BlobConvolution(x.permute(0, 2, 1, 3), f)                # not contiguous
+    with pytest.raises(AssertionError):
+        ops.BlobConvolution(x.double(), f)
+    with pytest.raises(AssertionError):
+        ops.BlobConvolution(x, torch.zeros(2, 3, 3, 5, device="cuda"))
+    with pytest.raises(ops.capi.Nb200Error):
+        ops.MultiplyMatrixByTransposedMatrix(x.view(25, 4), f.view(18, 4), first_row_size=3)
+    out = torch.empty(1, 3, 3, 2, device="cuda")
+    assert ops.BlobConvolution(x, f, result=out) is not None and torch.equal(out, y)
