@@ -68,19 +68,22 @@ __device__ __forceinline__ float lo_part(float v)
 	return v - __uint_as_float(__float_as_uint(v) & 0xffffe000u);
 }
 
-// ReLU (optionally with an upper threshold) and "no activation" as one clamp, HSwish apart; decided once per kernel
+// ReLU (optionally with an upper threshold) and "no activation" as one clamp, or HSwish.  Which of the two is a template
+// parameter: the depthwise warps apply it to 72 + 32 values per tile, and as a choice at run time both were computed.
+// (64 x 56 x 56, 32 -> 192 -> 32: 150.7 -> 148.5 us with the tests of interior tiles left out as well; the tile's period is
+// still set by the tensor-memory reads, the A operand's stores and the barrier.)
+template<bool HSWISH>
 struct Act {
-	bool hswish;
 	float lo, hi;
 	__device__ __forceinline__ float operator()(float v) const
 	{
-		return hswish ? v * fminf(fmaxf(v + 3.f, 0.f), 6.f) * (1.f / 6.f) : fminf(fmaxf(v, lo), hi);
+		return HSWISH ? v * fminf(fmaxf(v + 3.f, 0.f), 6.f) * (1.f / 6.f) : fminf(fmaxf(v, lo), hi);
 	}
 };
-__device__ __forceinline__ Act make_act(int kind, float param)
+template<bool HSWISH>
+__device__ __forceinline__ Act<HSWISH> make_act(int kind, float param)
 {
-	Act a;
-	a.hswish = kind == NB200_ACT_HSWISH;
+	Act<HSWISH> a;
 	a.lo = kind == NB200_ACT_RELU ? 0.f : -__int_as_float(0x7f800000);
 	a.hi = kind == NB200_ACT_RELU && param > 0.f ? param : __int_as_float(0x7f800000);
 	return a;
@@ -93,6 +96,11 @@ __device__ __forceinline__ void tmem_ld8_issue_local(uint32_t taddr, uint32_t* r
 		: "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
 		: "r"(taddr));
 }
+
+template<bool VALUE>
+struct Flag {
+	static constexpr bool value = VALUE;
+};
 
 struct SmemLayout {
 	uint32_t patchHi, patchLo, wExpHi, wExpLo, wDownHi, wDownLo, a2Hi, a2Lo, consts, bars, total;
@@ -123,7 +131,7 @@ __host__ __device__ inline SmemLayout smem_layout(int cExp, int cOut)
 	return l;
 }
 
-template<bool THREEX>
+template<bool THREEX, bool HSWISH_EXP, bool HSWISH_DW>
 __global__ void __launch_bounds__(THREADS, 1) mbv2_fused_kernel(const FusedParams p, const __grid_constant__ CUtensorMap mapX)
 {
 	extern __shared__ uint8_t smemRaw[];
@@ -191,7 +199,8 @@ __global__ void __launch_bounds__(THREADS, 1) mbv2_fused_kernel(const FusedParam
 	const uint32_t accProject = tmemBase + 4 * HALO_N;         // cOut columns; lanes 64..127 = the tile's 64 pixels
 	const uint32_t idescExpand = umma_idesc_tf32(128, HALO_N);
 	const uint32_t idescProject = umma_idesc_tf32(128, p.cOut);
-	const Act actExp = make_act(p.actExp, p.actExpParam), actDw = make_act(p.actDw, p.actDwParam);
+	const auto actExp = make_act<HSWISH_EXP>(p.actExp, p.actExpParam);
+	const auto actDw = make_act<HSWISH_DW>(p.actDw, p.actDwParam);
 
 	// Roles.  The lane quarter a warp may read (warp % 4) holds the 32 channels of chunk `combo`; a chunk has two
 	// depthwise warps, one per pair of output rows.  Quarters 2 and 3 exist only in the first 128-channel block: of
@@ -407,37 +416,40 @@ __global__ void __launch_bounds__(THREADS, 1) mbv2_fused_kernel(const FusedParam
 					rowBits[r] = (gy >= 0 && gy < p.h) ? colBits : 0u;
 				}
 				tmem_ld_wait();
-				float win[3][HW];
+				// The halo pixel's expanded value is zero outside the image.  A tile whose halo lies inside it (most tiles of a
+				// large image) runs the same arithmetic without the tests.
+				auto depthwise = [&](auto inside) {
+					auto expanded = [&](uint32_t bits, int r, int hx) {
+						const float v = actExp(__uint_as_float(bits) + biasExp);
+						return inside.value || ((rowBits[r] >> hx) & 1u) ? v : 0.f;
+					};
+					float win[3][HW];
 #pragma unroll
-				for(int r = 0; r < 3; ++r) {
+					for(int r = 0; r < 3; ++r) {
 #pragma unroll
-					for(int hx = 0; hx < HW; ++hx) {
-						const float v = actExp(__uint_as_float(raw[r * HW + hx]) + biasExp);
-						win[r][hx] = ((rowBits[r] >> hx) & 1u) ? v : 0.f;
+						for(int hx = 0; hx < HW; ++hx) win[r][hx] = expanded(raw[r * HW + hx], r, hx);
 					}
-				}
 #pragma unroll
-				for(int t = 0; t < 2; ++t) {
-					if(t == 1) {
-						// slide down: halo row 3 takes the place of halo row 0 (row index (t + dy) % 3 below)
+					for(int t = 0; t < 2; ++t) {
+						if(t == 1) {
+							// slide down: halo row 3 takes the place of halo row 0 (row index (t + dy) % 3 below)
 #pragma unroll
-						for(int hx = 0; hx < HW; ++hx) {
-							const uint32_t bits = hx < 16 ? last[hx] : last[16 + 6 + (hx - 16)];
-							const float v = actExp(__uint_as_float(bits) + biasExp);
-							win[0][hx] = ((rowBits[3] >> hx) & 1u) ? v : 0.f;
+							for(int hx = 0; hx < HW; ++hx) win[0][hx] = expanded(hx < 16 ? last[hx] : last[16 + 6 + (hx - 16)], 3, hx);
+						}
+#pragma unroll
+						for(int tx = 0; tx < TW; ++tx) {
+							float acc = biasDw;
+#pragma unroll
+							for(int dy = 0; dy < 3; ++dy) {
+#pragma unroll
+								for(int dx = 0; dx < 3; ++dx) acc = fmaf(win[(t + dy) % 3][tx + dx], k[dy * 3 + dx], acc);
+							}
+							out[t][tx] = actDw(acc);
 						}
 					}
-#pragma unroll
-					for(int tx = 0; tx < TW; ++tx) {
-						float acc = biasDw;
-#pragma unroll
-						for(int dy = 0; dy < 3; ++dy) {
-#pragma unroll
-							for(int dx = 0; dx < 3; ++dx) acc = fmaf(win[(t + dy) % 3][tx + dx], k[dy * 3 + dx], acc);
-						}
-						out[t][tx] = actDw(acc);
-					}
-				}
+				};
+				if((rowBits[0] & rowBits[1] & rowBits[2] & rowBits[3]) == (1u << HW) - 1u) depthwise(Flag<true>());
+				else depthwise(Flag<false>());
 				// project(j-1) still reads the A tiles when this tile's arithmetic is done early: wait, then write
 				if(j > 0) {
 					ok = mbar_wait_bounded(projectBar, (j - 1) & 1, abortFlag, p.status, (KERNEL_ID << 8) | SITE_PROJECT);
@@ -505,6 +517,24 @@ __global__ void __launch_bounds__(THREADS, 1) mbv2_fused_kernel(const FusedParam
 	if(warp == 0) tmem_dealloc(tmemBase, TMEM_COLS);
 }
 
+template<bool THREEX, bool HSWISH_EXP, bool HSWISH_DW>
+void launch_variant(const FusedParams& p, const CUtensorMap& map, int grid, size_t smemBytes, cudaStream_t stream)
+{
+	if(cudaFuncSetAttribute(mbv2_fused_kernel<THREEX, HSWISH_EXP, HSWISH_DW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+		static_cast<int>(smemBytes)) == cudaSuccess) {
+		mbv2_fused_kernel<THREEX, HSWISH_EXP, HSWISH_DW><<<grid, THREADS, smemBytes, stream>>>(p, map);
+	}
+}
+
+template<bool THREEX>
+void launch_kind(const FusedParams& p, const CUtensorMap& map, bool hsExp, bool hsDw, int grid, size_t smemBytes, cudaStream_t stream)
+{
+	if(hsExp && hsDw) launch_variant<THREEX, true, true>(p, map, grid, smemBytes, stream);
+	else if(hsExp) launch_variant<THREEX, true, false>(p, map, grid, smemBytes, stream);
+	else if(hsDw) launch_variant<THREEX, false, true>(p, map, grid, smemBytes, stream);
+	else launch_variant<THREEX, false, false>(p, map, grid, smemBytes, stream);
+}
+
 } // namespace
 
 // True when the block was issued as the fused kernel; false when the shape is outside what it covers (the caller then
@@ -535,14 +565,9 @@ bool launch_mbv2_fused(void* stream, const nb200_mbv2_desc* d, const float* x, c
 	CUtensorMap map;
 	if(!make_image_box_map(&map, x, CIN, d->w, d->h, d->batch, CIN, HW, HH, 1)) return false;
 	const int grid = p.numTiles < sm_count() ? p.numTiles : sm_count();
-	cudaError_t e;
-	if(precision == NB200_PREC_3XTF32) {
-		e = cudaFuncSetAttribute(mbv2_fused_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smemBytes));
-		if(e == cudaSuccess) mbv2_fused_kernel<true><<<grid, THREADS, smemBytes, as_stream(stream)>>>(p, map);
-	} else {
-		e = cudaFuncSetAttribute(mbv2_fused_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smemBytes));
-		if(e == cudaSuccess) mbv2_fused_kernel<false><<<grid, THREADS, smemBytes, as_stream(stream)>>>(p, map);
-	}
+	const bool hsExp = d->act_exp == NB200_ACT_HSWISH, hsDw = d->act_dw == NB200_ACT_HSWISH;
+	if(precision == NB200_PREC_3XTF32) launch_kind<true>(p, map, hsExp, hsDw, grid, smemBytes, as_stream(stream));
+	else launch_kind<false>(p, map, hsExp, hsDw, grid, smemBytes, as_stream(stream));
 	count_launch(1);
 	*rc = check_launch();
 	return true;
