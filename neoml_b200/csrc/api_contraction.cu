@@ -135,14 +135,14 @@ size_t prepared_filter_floats(long long k, long long r, long long s, long long c
 }
 
 // Whether a launch of this many 128-row tiles, n columns and depth k goes to the fp16 kernel (3xTF32 accuracy,
-// contraction_split.cu) when its second operand is prepared: from the tile count on that no longer splits K, i.e. where
-// throughput and not the length of one tile's K loop decides (below it the TF32 kernel with split K stays), and from five
-// K blocks on (a shorter loop is hidden behind its epilogue; ResNet-50 at batch 256, TF32 against fp16 kernel: K = 64 and
-// 128 with residual 355 / 430 us and 197 / 239, K = 256 158 / 150, K = 1152 284 / 195).
+// contraction_split.cu) when its second operand is prepared.  From the tile count on that no longer splits K it does so
+// from five K blocks on (a shorter loop is hidden behind its epilogue; ResNet-50 at batch 256, TF32 against fp16 kernel: K =
+// 64 and 128 with residual 355 / 430 us and 197 / 239, K = 256 158 / 150, K = 1152 284 / 195).  With fewer tiles a launch is
+// a few K blocks per part and a finishing pass in either kernel: it does from 32 K blocks on.
 bool split_form_pays(long long mTiles, long long n, long long k, long long batch)
 {
 	const int width = contraction_tile_width(static_cast<int>(n));
-	return k > 128 && mTiles * ((n + width - 1) / width) * batch > SPLIT_TILES_MAX;
+	return k > (mTiles * ((n + width - 1) / width) * batch > SPLIT_TILES_MAX ? 128 : 1023);
 }
 
 // Row-window form of a convolution with few channels (the network stem): the image is copied once with its spatial
@@ -428,6 +428,7 @@ static int matrix_product(void* stream, int batch, const float* a, int m, int k,
 		const int rc = split_operand(b, rows, ldb, k, rest, as_stream(stream));
 		if(rc != NB200_OK) return rc;
 		set_split_operand(p, rest, rows, k);
+		rest += split_operand_floats(rows, k);
 	} else if(prepare) {
 		// one pass over the second operand as it lies in memory (the floats between its rows, if any, are carried along)
 		if(device_status_word() == nullptr) return NB200_ENODEVICE;
@@ -684,11 +685,12 @@ int blob_convolution(void* stream, const nb200_conv_desc* d, const float* x, con
 		// with few output rows (small batches) every filter tile is used by a handful of CTAs at most: the extra launch
 		// costs more than converting those tiles in the kernel (ResNet-50 at batch 1: 0.69 -> 0.62 ms per pass)
 		const bool prepare = outRows >= PREPARE_B_MIN_ROWS;
+		bool split = false;
 		if(prepare) {
 			const bool given = prepared != nullptr && aligned16(prepared);
 			// the fp16 kernel's form where the launch is large enough; a caller whose room (a fixed array) is too small
 			// for its scales keeps the TF32 kernel
-			const bool split = precision == NB200_PREC_3XTF32 && split_form_pays(d, false)
+			split = precision == NB200_PREC_3XTF32 && split_form_pays(d, false)
 				&& (given || scratchFloats >= static_cast<size_t>(inScratch - scratch) + split_operand_floats(d->k, kk));
 			const float* ready = given ? prepared + (split ? prepared_filter_floats(d->k, d->r, d->s, d->c) : 0) : nullptr;
 			if(ready == nullptr && split) {
@@ -710,7 +712,7 @@ int blob_convolution(void* stream, const nb200_conv_desc* d, const float* x, con
 			p.b_ready = 1;
 		}
 		// whatever the caller's scratch holds beyond the prepared filter is room for split-K partial results
-		float* const rest = inScratch + prepared_filter_floats(d->k, d->r, d->s, d->c);
+		float* const rest = inScratch + (split ? split_operand_floats(d->k, kk) : prepared_filter_floats(d->k, d->r, d->s, d->c));
 		const size_t used = static_cast<size_t>(rest - scratch);
 		if(scratchFloats > used + 4 && split_scratch_floats(outRows, d->k, kk) > 0) {
 			p.splitScratch = rest;

@@ -122,6 +122,22 @@ int balanced_tile_width(long long mTiles, int n, int batch);
 // Tensor maps (CUtensorMap behind the void pointer), contraction_tc.cu
 bool make_rows_map(void* map, const float* base, int k, long long rows, long long ld, int batch, long long batchStride, int boxRows);
 int make_operand_map(void* map, const ContractionParams& p, int batch, int boxRows);
+// Tail of a split-K launch: out = act(part 0 + part 1 + ... (in this order) + bias[n] + residual[m][n]).
+struct SplitFinish {
+	float* out;
+	int parts;
+	long long slab; // floats per part
+	const float* bias;
+	const float* residual;
+	int ldr;
+	int act;
+	float actParam;
+	const float* actParamDevice;
+};
+// Decides on split K for a launch of numTiles tiles fed by TMA: sets p.kSplits, and where that is more than one redirects
+// p's output to the scratch and takes the epilogue out of p.
+SplitFinish split_k(ContractionParams& p, long long numTiles, int numKb, int batch);
+void launch_split_finish(const ContractionParams& p, const SplitFinish& finish, cudaStream_t stream);
 bool timing_events(cudaEvent_t* start, cudaEvent_t* stop);
 // The split form of a [rows x k] operand (rows `ld` floats apart, 16-byte aligned): floats it
 // takes, and the kernel that makes it; the row scales follow the rows at rows * (k rounded up to 32).

@@ -165,7 +165,9 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 	constexpr int HALF_COLS = BN / 2;
 	constexpr int CHUNKS = HALF_COLS / 16;
 
-	const int numKb = (p.K + BK - 1) / BK;
+	// with split K the unit of work is (tile, K part): `numTiles` counts those, each covers numKb K blocks
+	const int kSplits = p.kSplits;
+	const int numKb = ((p.K + BK - 1) / BK) / kSplits;
 	constexpr int SLOT_BYTES = A_TILE_BYTES + B_TILE_BYTES;
 
 	uint8_t* rawRing = smem;
@@ -231,7 +233,9 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 		bool ok = true;
 		const int hw = p.Ho * p.Wo;
 		for(int local = 0; local < myTiles && ok; ++local, tile += gridDim.x) {
-			const TileCoord tc = tile_coord(tile, nTiles, tilesPerBatch, BN, p.tileM);
+			const int tileIdx = tile / kSplits;
+			const int kbBegin = (tile - tileIdx * kSplits) * numKb;
+			const TileCoord tc = tile_coord(tileIdx, nTiles, tilesPerBatch, BN, p.tileM);
 			int w0 = 0, h0 = 0, img = 0;
 			if(p.a_tma == 3) {
 				const int outRow = tc.m0 / p.tileM; // = image * Ho + oy
@@ -245,7 +249,13 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 				h0 = oy * p.strH - p.padH;
 			}
 			int c0 = 0, fs = 0, fr = 0; // channel offset inside the filter tap, tap column, tap row
-			for(int kb = 0; kb < numKb; ++kb) {
+			if(p.a_tma == 2 && kbBegin > 0) {
+				const int tap = kbBegin * BK / p.Cin;
+				c0 = kbBegin * BK - tap * p.Cin;
+				fr = tap / p.S;
+				fs = tap - fr * p.S;
+			}
+			for(int kb = kbBegin; kb < kbBegin + numKb; ++kb) {
 				if(!mbar_wait_bounded_warp(&rawEmptyBar[slot], parity, abortFlag, p.status, SITE_RAW_EMPTY)) { ok = false; break; }
 				const uint32_t aTile = smem_u32(rawRing + static_cast<size_t>(slot) * SLOT_BYTES);
 				if(elect_one()) {
@@ -282,13 +292,14 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 			const uint32_t accMain = tmemBase + set * BN;
 			const uint32_t accCross = tmemBase + CROSS_BASE + (FOLD ? 0 : set * BN);
 			uint32_t acc = 0u; // the first products of a tile overwrite the accumulators
+			const int kbBegin = (blockIdx.x + local * gridDim.x) % kSplits * numKb;
 			for(int kb = 0; kb < numKb; ++kb) {
 				if(!mbar_wait_bounded_warp(&cvtFullBar[stage], stageParity, abortFlag, p.status, SITE_CVT_FULL)) { ok = false; break; }
 				tc_fence_after_sync();
 				const uint32_t aHi = tmemBase + A_BASE + stage * STAGE_COLS, aLo = aHi + 8;
 				const uint32_t bTile = smem_u32(rawRing + static_cast<size_t>(slot) * SLOT_BYTES) + A_TILE_BYTES;
 				const uint64_t dB = umma_desc_k128(bTile); // 16 halves = 32 bytes = +2; the lo halves start 64 bytes in
-				const bool both = p.K - kb * BK > 16;
+				const bool both = p.K - (kbBegin + kb) * BK > 16;
 				if(elect_one()) {
 					umma_f16_ts(accCross, aLo, dB, idesc, acc);
 					umma_f16_ts(accMain, aHi, dB, idesc, acc);
@@ -425,8 +436,11 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 		bool ok = true;
 		int ring = 0;
 		for(int local = 0; local < myTiles && ok; ++local) {
-			const TileCoord tc = tile_coord(blockIdx.x + local * gridDim.x, nTiles, tilesPerBatch, BN, p.tileM);
-			float* __restrict__ C = p.C + tc.batch * p.strideC;
+			const int work = blockIdx.x + local * gridDim.x;
+			const int tileIdx = work / kSplits;
+			const TileCoord tc = tile_coord(tileIdx, nTiles, tilesPerBatch, BN, p.tileM);
+			// a K part of a split launch stores its partial sums in its own slab
+			float* __restrict__ C = p.C + tc.batch * p.strideC + static_cast<size_t>(work - tileIdx * kSplits) * p.M * p.ldc;
 			const float* __restrict__ R = p.residual != nullptr ? p.residual + tc.batch * p.strideC : nullptr;
 			const int set = local & 1;
 			const uint32_t accParity = (local >> 1) & 1;
@@ -749,7 +763,9 @@ int launch_bn(const ContractionParams& p0, int batch, cudaStream_t stream)
 		static_cast<long long>(p.N) * packedRow, BN)) {
 		return NB200_EINVAL;
 	}
-	const int grid = numTiles < sms ? static_cast<int>(numTiles) : sms;
+	const SplitFinish finish = split_k(p, numTiles, numKb, batch);
+	const long long numWork = numTiles * p.kSplits;
+	const int grid = numWork < sms ? static_cast<int>(numWork) : sms;
 	// as many raw slots as fit the 227 KB a CTA may use: the copies run that many K blocks ahead
 	constexpr int fixedBytes = EPI_WARPS * STAGING_BYTES_PER_WARP + EPI_WARPS * BN * 4 /*strips*/ + (SCALE_RING + 1) * BM * 4
 		+ 512 /*barriers*/ + 1024 /*alignment slack*/;
@@ -757,13 +773,14 @@ int launch_bn(const ContractionParams& p0, int batch, cudaStream_t stream)
 	constexpr int fitting = (227 * 1024 - fixedBytes) / slotBytes;
 	constexpr int rawSlots = fitting < MAX_RAW_SLOTS ? fitting : MAX_RAW_SLOTS;
 	constexpr size_t smemBytes = static_cast<size_t>(rawSlots) * slotBytes + fixedBytes;
-	const int nt = static_cast<int>(numTiles), nn = static_cast<int>(nTiles), tpb = static_cast<int>(tilesPerBatch);
+	const int nt = static_cast<int>(numWork), nn = static_cast<int>(nTiles), tpb = static_cast<int>(tilesPerBatch);
 	cudaEvent_t timedStart = nullptr, timedStop = nullptr;
 	const bool timed = timing_events(&timedStart, &timedStop);
 	if(timed) cudaEventRecord(timedStart, stream);
 	const bool overlap = overlap_launches();
 	launch_dependent(overlap, contraction_split_kernel<BN>, dim3(grid), dim3(THREADS), smemBytes, stream, p, nt, nn, tpb, rawSlots, mapA, mapB);
 	count_launch();
+	if(p.kSplits > 1) launch_split_finish(p, finish, stream);
 	if(timed) cudaEventRecord(timedStop, stream);
 	return check_launch();
 }
@@ -789,7 +806,8 @@ int launch_contraction_split(const ContractionParams& p, int batch, cudaStream_t
 {
 	if(p.M <= 0 || p.N <= 0 || batch <= 0) return NB200_OK;
 	const int tileM = p.a_mode == A_CONV_WINDOW && p.tileM > 0 && p.tileM <= BM ? p.tileM : BM;
-	switch(balanced_tile_width((p.M + tileM - 1LL) / tileM, p.N, batch)) {
+	const bool maySplit = p.splitScratch != nullptr && batch == 1 && p.K >= 8 * BK;
+	switch(maySplit ? contraction_tile_width(p.N) : balanced_tile_width((p.M + tileM - 1LL) / tileM, p.N, batch)) {
 		case 32: return launch_bn<32>(p, batch, stream);
 		case 64: return launch_bn<64>(p, batch, stream);
 		case 96: return launch_bn<96>(p, batch, stream);

@@ -1017,19 +1017,6 @@ bool make_image_box_map(void* map, const float* base, int c, int w, int h, int n
 
 namespace {
 
-// Tail of a split-K launch: out = act(part 0 + part 1 + ... (in this order) + bias[n] + residual[m][n]).
-struct SplitFinish {
-	float* out;
-	int parts;
-	long long slab; // floats per part
-	const float* bias;
-	const float* residual;
-	int ldr;
-	int act;
-	float actParam;
-	const float* actParamDevice;
-};
-
 __global__ void __launch_bounds__(256) split_finish_kernel(const float* __restrict__ partials, int n4, long long quads,
 	const SplitFinish f)
 {
@@ -1161,29 +1148,11 @@ int launch_bn(const ContractionParams& p0, int batch, cudaStream_t stream)
 		return NB200_EINVAL;
 	}
 	const bool gather = p.a_tma == 0 || p.b_tma == 0;
-	// Few tiles and a long K loop (small batches: a handful of CTAs would walk dozens of K blocks while the other SMs
-	// idle): cut every tile's K loop into equal parts that run as separate work items and store their partial sums in
-	// slabs of the caller's scratch; a finishing pass sums the slabs in order and applies bias, residual, activation.
 	const int numKb = (p.K + BK - 1) / BK;
-	int kSplits = 1;
-	const long long slab = static_cast<long long>(p.M) * p.N;
-	if(!gather && numTiles * 2 <= sms && numKb >= 8 && p.c_vec && !p.accumulate && batch == 1 && p.ldc == p.N
-		&& p.splitScratch != nullptr && aligned16(p.splitScratch) && !(g_traceOptions & 32)) {
-		const long long room = sms / numTiles;
-		// at least four K blocks per part (measured: two is no better, eight is slower at batch 1)
-		for(int d = 2; d <= numKb / 4 && d <= room && d * slab <= p.splitScratchFloats; ++d) {
-			if(numKb % d == 0) kSplits = d; // the largest divisor of the K-block count that fits the machine and the scratch
-		}
-	}
 	SplitFinish finish = {};
-	if(kSplits > 1) {
-		finish.bias = p.bias; finish.residual = p.residual; finish.ldr = p.ldr; finish.act = p.act; finish.actParam = p.act_param;
-		finish.actParamDevice = p.act_param_device;
-		finish.out = p.C; finish.parts = kSplits; finish.slab = slab;
-		p.bias = nullptr; p.residual = nullptr; p.act = NB200_ACT_NONE; p.act_param_device = nullptr;
-		p.C = p.splitScratch;
-	}
-	p.kSplits = kSplits;
+	p.kSplits = 1;
+	if(!gather) finish = split_k(p, numTiles, numKb, batch);
+	const int kSplits = p.kSplits;
 	const long long numWork = numTiles * kSplits;
 	int grid = numWork < sms ? static_cast<int>(numWork) : sms;
 	// Short K loops with a prepared B: keep the CTA's B columns (all K blocks, hi + lo) in shared memory for all of its
@@ -1231,17 +1200,47 @@ int launch_bn(const ContractionParams& p0, int batch, cudaStream_t stream)
 	}
 #undef NB200_LAUNCH
 	count_launch();
-	if(kSplits > 1) {
-		const long long quads = slab / 4;
-		launch_dependent(overlap, split_finish_kernel, dim3(grid_for(quads, 256, 16)), dim3(256), 0, stream,
-			static_cast<const float*>(p.splitScratch), p.N / 4, quads, finish);
-		count_launch();
-	}
+	if(kSplits > 1) launch_split_finish(p, finish, stream);
 	if(timed) cudaEventRecord(timedStop, stream);
 	return check_launch();
 }
 
 } // namespace
+
+// Few tiles and a long K loop (small batches: a handful of CTAs would walk dozens of K blocks while the other SMs idle): cut
+// every tile's K loop into equal parts that run as separate work items and store their partial sums in slabs of the
+// caller's scratch; a finishing pass sums the slabs in order and applies bias, residual, activation.
+SplitFinish split_k(ContractionParams& p, long long numTiles, int numKb, int batch)
+{
+	SplitFinish finish = {};
+	p.kSplits = 1;
+	const int sms = sm_count();
+	const long long slab = static_cast<long long>(p.M) * p.N;
+	if(numTiles * 2 <= sms && numKb >= 8 && p.c_vec && !p.accumulate && batch == 1 && p.ldc == p.N
+		&& p.splitScratch != nullptr && aligned16(p.splitScratch) && !(g_traceOptions & 32)) {
+		const long long room = sms / numTiles;
+		// at least four K blocks per part (measured: two is no better, eight is slower at batch 1)
+		for(int d = 2; d <= numKb / 4 && d <= room && d * slab <= p.splitScratchFloats; ++d) {
+			if(numKb % d == 0) p.kSplits = d; // the largest divisor of the K-block count that fits the machine and the scratch
+		}
+	}
+	if(p.kSplits > 1) {
+		finish.bias = p.bias; finish.residual = p.residual; finish.ldr = p.ldr; finish.act = p.act; finish.actParam = p.act_param;
+		finish.actParamDevice = p.act_param_device;
+		finish.out = p.C; finish.parts = p.kSplits; finish.slab = slab;
+		p.bias = nullptr; p.residual = nullptr; p.act = NB200_ACT_NONE; p.act_param_device = nullptr;
+		p.C = p.splitScratch;
+	}
+	return finish;
+}
+
+void launch_split_finish(const ContractionParams& p, const SplitFinish& finish, cudaStream_t stream)
+{
+	const long long quads = finish.slab / 4;
+	launch_dependent(overlap_launches(), split_finish_kernel, dim3(grid_for(quads, 256, 16)), dim3(256), 0, stream,
+		static_cast<const float*>(p.splitScratch), p.N / 4, quads, finish);
+	count_launch();
+}
 
 void time_contractions(bool enable)
 {
