@@ -9,7 +9,24 @@ namespace nb200 {
 enum { A_ROWS = 0, A_CONV_TAP = 1, A_CONV_WINDOW = 2 };
 enum { B_ROWS = 0, B_COLS = 1 };
 
+// Division of a non-negative int by a divisor known at launch: a multiplication and a shift (Granlund and Montgomery,
+// "Division by invariant integers using multiplication", 1994) in place of some forty dependent instructions.  A tile's
+// coordinates take three to five of them, one after the other, in the warp that has the next copy to issue: 1300 cycles.
+struct FastDiv {
+	uint32_t mul;
+	int shift;
+	__device__ __forceinline__ int operator()(int n) const
+	{
+		return static_cast<int>((__umulhi(static_cast<uint32_t>(n), mul) + static_cast<uint32_t>(n)) >> shift);
+	}
+};
+FastDiv fast_div(long long d); // 1 <= d < 2^31
+struct TileDivs {
+	FastDiv splits, perBatch, nTiles, ho, hw, wo;
+};
+
 struct ContractionParams {
+	TileDivs div; // set by the launcher
 	const float* A;
 	const float* B;
 	float* C;
@@ -60,6 +77,21 @@ struct ContractionParams {
 	unsigned long long* trace;
 	int traceSteps;
 };
+
+struct TileCoord {
+	int m0, n0, batch, mTile;
+};
+
+__device__ __forceinline__ TileCoord tile_coord(const ContractionParams& p, int tile, int nTiles, int tilesPerBatch, int bn)
+{
+	TileCoord t;
+	t.batch = p.div.perBatch(tile);
+	const int r = tile - t.batch * tilesPerBatch;
+	t.mTile = p.div.nTiles(r);
+	t.m0 = t.mTile * p.tileM;
+	t.n0 = (r - t.mTile * nTiles) * bn;
+	return t;
+}
 
 // Decodes output row m of a convolution into the image base offset and the top-left input coordinate.
 struct ConvRow {
@@ -116,6 +148,7 @@ __device__ __forceinline__ float gather_b(const ContractionParams& p, const floa
 
 void set_contraction_trace(unsigned long long* buffer, int steps, int options);
 int launch_contraction_tc(const ContractionParams& p, int batch, cudaStream_t stream);
+TileDivs tile_divs(const ContractionParams& p, long long nTiles, long long tilesPerBatch);
 int launch_contraction_split(const ContractionParams& p, int batch, cudaStream_t stream);
 int contraction_tile_width(int n);
 int balanced_tile_width(long long mTiles, int n, int batch);

@@ -23,8 +23,10 @@
 // to reach the result (a row of 1e6 and 1e-6 times weights of 1e-6 and 1e6: 1e-4).
 //
 // Pipeline: as in contraction_tc.cu, a persistent CTA per SM (24 warps) walks the 128 x BN tiles:
-//   warp 0       copies by TMA into a ring of raw slots: A (128 rows x 32 floats; plain rows, im2col or row windows) and B
-//                (BN rows x 128 bytes: 32 hi halves, 32 lo halves)
+//   warps 0, 1   copy by TMA into a ring of raw slots: A (128 rows x 32 floats; plain rows, im2col or row windows) and B
+//                (BN rows x 128 bytes: 32 hi halves, 32 lo halves), a warp each: a wait, an announcement and two copies took
+//                one warp about as long (640 cycles) as the block's conversion (3x3 64 -> 64, 32 x 56 x 56: 54.5 us with one
+//                copy warp and tile coordinates by division, 50.9 now)
 //   warps 4-15   convert, three groups of four warps that take the K blocks in turn, each with a stage of its own in tensor
 //                memory (32 columns); thread = row of the tile.  The row scales go from group to group in shared memory:
 //                a group looks at its block's maxima, waits for the scales after the block before, publishes its own and
@@ -82,21 +84,6 @@ enum {
 __device__ __forceinline__ uint32_t swz(int row, int chunk)
 {
 	return static_cast<uint32_t>(row) * 128u + (static_cast<uint32_t>(chunk ^ (row & 7)) << 4);
-}
-
-struct TileCoord {
-	int m0, n0, batch;
-};
-
-__device__ __forceinline__ TileCoord tile_coord(int tile, int nTiles, int tilesPerBatch, int bn, int tileM)
-{
-	TileCoord t;
-	t.batch = tile / tilesPerBatch;
-	const int r = tile - t.batch * tilesPerBatch;
-	const int mTile = r / nTiles;
-	t.m0 = mTile * tileM;
-	t.n0 = (r - mTile * nTiles) * bn;
-	return t;
 }
 
 // The power of two that puts `largest` into [2^TARGET_EXP, 2^(TARGET_EXP + 1)), kept where it and its inverse are
@@ -193,7 +180,7 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 
 	if(tid == 0) {
 		for(int s = 0; s < MAX_RAW_SLOTS; ++s) {
-			mbar_init(&rawFullBar[s], 1);
+			mbar_init(&rawFullBar[s], 2); // one announcement per copy warp
 			mbar_init(&rawEmptyBar[s], 1);
 		}
 		for(int s = 0; s < STAGES; ++s) mbar_init(&cvtFullBar[s], CVT_WARPS);
@@ -226,25 +213,24 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 	if(warp < CVT_WARP0) {
 		registers_down<REGS_ISSUE>();
 		if(warp == 0) {
-		// ------------------------------------------------------------------ copy
+		// ------------------------------------------------------------------ copy A
 		int tile = blockIdx.x;
 		int slot = 0;
 		uint32_t parity = 1; // the first pass over the ring finds every slot free
 		bool ok = true;
 		const int hw = p.Ho * p.Wo;
 		for(int local = 0; local < myTiles && ok; ++local, tile += gridDim.x) {
-			const int tileIdx = tile / kSplits;
+			const int tileIdx = p.div.splits(tile);
 			const int kbBegin = (tile - tileIdx * kSplits) * numKb;
-			const TileCoord tc = tile_coord(tileIdx, nTiles, tilesPerBatch, BN, p.tileM);
+			const TileCoord tc = tile_coord(p, tileIdx, nTiles, tilesPerBatch, BN);
 			int w0 = 0, h0 = 0, img = 0;
 			if(p.a_tma == 3) {
-				const int outRow = tc.m0 / p.tileM; // = image * Ho + oy
-				img = outRow / p.Ho;
-				h0 = outRow - img * p.Ho;
+				img = p.div.ho(tc.mTile); // the tile is output row image * Ho + oy
+				h0 = tc.mTile - img * p.Ho;
 			} else if(p.a_tma == 2) {
-				img = tc.m0 / hw;
+				img = p.div.hw(tc.m0);
 				const int rem = tc.m0 - img * hw;
-				const int oy = rem / p.Wo;
+				const int oy = p.div.wo(rem);
 				w0 = (rem - oy * p.Wo) * p.strW - p.padW;
 				h0 = oy * p.strH - p.padH;
 			}
@@ -259,7 +245,7 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 				if(!mbar_wait_bounded_warp(&rawEmptyBar[slot], parity, abortFlag, p.status, SITE_RAW_EMPTY)) { ok = false; break; }
 				const uint32_t aTile = smem_u32(rawRing + static_cast<size_t>(slot) * SLOT_BYTES);
 				if(elect_one()) {
-					mbar_arrive_expect_tx(&rawFullBar[slot], SLOT_BYTES);
+					mbar_arrive_expect_tx(&rawFullBar[slot], A_TILE_BYTES);
 					if(p.a_tma == 1) {
 						tma_load_3d(aTile, &mapA, &rawFullBar[slot], kb * BK, tc.m0, tc.batch);
 					} else if(p.a_tma == 3) {
@@ -268,13 +254,32 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 						tma_load_im2col_4d(aTile, &mapA, &rawFullBar[slot], c0, w0, h0, img,
 							static_cast<uint16_t>(fs * p.dilW), static_cast<uint16_t>(fr * p.dilH));
 					}
-					tma_load_3d(aTile + A_TILE_BYTES, &mapB, &rawFullBar[slot], kb * BK, tc.n0, tc.batch);
 				}
 				__syncwarp();
 				if(p.a_tma == 2) {
 					c0 += BK;
 					if(c0 >= p.Cin) { c0 = 0; if(++fs == p.S) { fs = 0; ++fr; } }
 				}
+				if(++slot == rawSlots) { slot = 0; parity ^= 1; }
+			}
+		}
+		} else if(warp == 1) {
+		// ------------------------------------------------------------------ copy B
+		int slot = 0;
+		uint32_t parity = 1;
+		bool ok = true;
+		for(int local = 0, tile = blockIdx.x; local < myTiles && ok; ++local, tile += gridDim.x) {
+			const int tileIdx = p.div.splits(tile);
+			const int kbBegin = (tile - tileIdx * kSplits) * numKb;
+			const TileCoord tc = tile_coord(p, tileIdx, nTiles, tilesPerBatch, BN);
+			for(int kb = kbBegin; kb < kbBegin + numKb; ++kb) {
+				if(!mbar_wait_bounded_warp(&rawEmptyBar[slot], parity, abortFlag, p.status, SITE_RAW_EMPTY)) { ok = false; break; }
+				if(elect_one()) {
+					mbar_arrive_expect_tx(&rawFullBar[slot], B_TILE_BYTES);
+					tma_load_3d(smem_u32(rawRing + static_cast<size_t>(slot) * SLOT_BYTES) + A_TILE_BYTES, &mapB, &rawFullBar[slot],
+						kb * BK, tc.n0, tc.batch);
+				}
+				__syncwarp();
 				if(++slot == rawSlots) { slot = 0; parity ^= 1; }
 			}
 		}
@@ -292,7 +297,8 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 			const uint32_t accMain = tmemBase + set * BN;
 			const uint32_t accCross = tmemBase + CROSS_BASE + (FOLD ? 0 : set * BN);
 			uint32_t acc = 0u; // the first products of a tile overwrite the accumulators
-			const int kbBegin = (blockIdx.x + local * gridDim.x) % kSplits * numKb;
+			const int work = blockIdx.x + local * gridDim.x;
+			const int kbBegin = kSplits == 1 ? 0 : (work - p.div.splits(work) * kSplits) * numKb;
 			for(int kb = 0; kb < numKb; ++kb) {
 				if(!mbar_wait_bounded_warp(&cvtFullBar[stage], stageParity, abortFlag, p.status, SITE_CVT_FULL)) { ok = false; break; }
 				tc_fence_after_sync();
@@ -437,8 +443,8 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 		int ring = 0;
 		for(int local = 0; local < myTiles && ok; ++local) {
 			const int work = blockIdx.x + local * gridDim.x;
-			const int tileIdx = work / kSplits;
-			const TileCoord tc = tile_coord(tileIdx, nTiles, tilesPerBatch, BN, p.tileM);
+			const int tileIdx = p.div.splits(work);
+			const TileCoord tc = tile_coord(p, tileIdx, nTiles, tilesPerBatch, BN);
 			// a K part of a split launch stores its partial sums in its own slab
 			float* __restrict__ C = p.C + tc.batch * p.strideC + static_cast<size_t>(work - tileIdx * kSplits) * p.M * p.ldc;
 			const float* __restrict__ R = p.residual != nullptr ? p.residual + tc.batch * p.strideC : nullptr;
@@ -773,6 +779,7 @@ int launch_bn(const ContractionParams& p0, int batch, cudaStream_t stream)
 	constexpr int fitting = (227 * 1024 - fixedBytes) / slotBytes;
 	constexpr int rawSlots = fitting < MAX_RAW_SLOTS ? fitting : MAX_RAW_SLOTS;
 	constexpr size_t smemBytes = static_cast<size_t>(rawSlots) * slotBytes + fixedBytes;
+	p.div = tile_divs(p, nTiles, tilesPerBatch);
 	const int nt = static_cast<int>(numWork), nn = static_cast<int>(nTiles), tpb = static_cast<int>(tilesPerBatch);
 	cudaEvent_t timedStart = nullptr, timedStop = nullptr;
 	const bool timed = timing_events(&timedStart, &timedStop);

@@ -93,21 +93,6 @@ __device__ __forceinline__ void trace(const ContractionParams& p, int role, int 
 	if(p.trace != nullptr && blockIdx.x == 0 && step < p.traceSteps) p.trace[role * p.traceSteps + step] = clock64();
 }
 
-struct TileCoord {
-	int m0, n0, batch;
-};
-
-__device__ __forceinline__ TileCoord tile_coord(int tile, int nTiles, int tilesPerBatch, int bn, int tileM)
-{
-	TileCoord t;
-	t.batch = tile / tilesPerBatch;
-	const int r = tile - t.batch * tilesPerBatch;
-	const int mTile = r / nTiles;
-	t.m0 = mTile * tileM;
-	t.n0 = (r - mTile * nTiles) * bn;
-	return t;
-}
-
 // GATHER = false: both operands arrive by TMA and the cp.async gather code (with its per-row bookkeeping registers) is
 // not even compiled in; GATHER = true: the general kernel.
 // BRES = true (all-TMA only): the variant for short K loops, where a tile's epilogue outlasts its main loop.  The
@@ -240,7 +225,7 @@ __global__ void __maxnreg__(128) contraction_tc_kernel(const ContractionParams p
 			const int hw = p.Ho * p.Wo;
 			if(bRes && myTiles > 0) {
 				// all K blocks of this CTA's B columns, once
-				const TileCoord first = tile_coord(blockIdx.x, nTiles, tilesPerBatch, BN, p.tileM);
+				const TileCoord first = tile_coord(p, blockIdx.x, nTiles, tilesPerBatch, BN);
 				if(elect_one()) {
 					mbar_arrive_expect_tx(bResidentBar, static_cast<uint32_t>(numKb * B_STEP_BYTES));
 					for(int kb = 0; kb < numKb; ++kb) {
@@ -252,18 +237,17 @@ __global__ void __maxnreg__(128) contraction_tc_kernel(const ContractionParams p
 				__syncwarp();
 			}
 			for(int local = 0; local < myTiles && ok; ++local, tile += gridDim.x) {
-				const int tileIdx = tile / kSplits;
+				const int tileIdx = p.div.splits(tile);
 				const int kbBegin = (tile - tileIdx * kSplits) * kbPer;
-				const TileCoord tc = tile_coord(tileIdx, nTiles, tilesPerBatch, BN, p.tileM);
+				const TileCoord tc = tile_coord(p, tileIdx, nTiles, tilesPerBatch, BN);
 				int w0 = 0, h0 = 0, img = 0;
 				if(p.a_tma == 3) {
-					const int outRow = tc.m0 / p.tileM; // = image * Ho + oy
-					img = outRow / p.Ho;
-					h0 = outRow - img * p.Ho;
+					img = p.div.ho(tc.mTile); // the tile is output row image * Ho + oy
+					h0 = tc.mTile - img * p.Ho;
 				} else if(p.a_tma == 2) {
-					img = tc.m0 / hw;
+					img = p.div.hw(tc.m0);
 					const int rem = tc.m0 - img * hw;
-					const int oy = rem / p.Wo;
+					const int oy = p.div.wo(rem);
 					w0 = (rem - oy * p.Wo) * p.strW - p.padW;
 					h0 = oy * p.strH - p.padH;
 				}
@@ -316,7 +300,7 @@ __global__ void __maxnreg__(128) contraction_tc_kernel(const ContractionParams p
 		int step = 0;
 		bool ok = true;
 		for(int local = 0; local < myTiles && ok; ++local, tile += gridDim.x) {
-			const TileCoord tc = tile_coord(tile, nTiles, tilesPerBatch, BN, p.tileM);
+			const TileCoord tc = tile_coord(p, tile, nTiles, tilesPerBatch, BN);
 			const float* A = p.A + tc.batch * p.strideA;
 			const float* B = p.B + tc.batch * p.strideB;
 			// where this thread's rows start: an element offset into A (row-major) or the image origin (convolution)
@@ -561,7 +545,7 @@ __global__ void __maxnreg__(128) contraction_tc_kernel(const ContractionParams p
 				const uint32_t accCross = SEP_CROSS ? tmemBase + CROSS_BASE + (FOLD ? 0 : set * ACC_COLS) : accMain;
 				uint32_t acc = 0u; // the first MMA of a tile overwrites the accumulators
 				const int work = blockIdx.x + local * gridDim.x;
-				const int kbBegin = (work % kSplits) * kbPer;
+				const int kbBegin = kSplits == 1 ? 0 : (work - p.div.splits(work) * kSplits) * kbPer;
 				for(int kb = kbBegin; kb < kbBegin + kbPer; ++kb, ++it) {
 					const int ls = it % LO_SLOTS;
 					if(!mbar_wait_bounded_warp(&cvtFullBar[ls], (it / LO_SLOTS) & 1, abortFlag, p.status, SITE_CVT_FULL)) { ok = false; break; }
@@ -638,8 +622,8 @@ __global__ void __maxnreg__(128) contraction_tc_kernel(const ContractionParams p
 		bool ok = true;
 		for(int local = 0; local < myTiles && ok; ++local) {
 			const int work = blockIdx.x + local * gridDim.x;
-			const int tile = work / kSplits;
-			const TileCoord tc = tile_coord(tile, nTiles, tilesPerBatch, BN, p.tileM);
+			const int tile = p.div.splits(work);
+			const TileCoord tc = tile_coord(p, tile, nTiles, tilesPerBatch, BN);
 			// a K part of a split launch stores its partial sums in its own slab
 			float* __restrict__ C = p.C + tc.batch * p.strideC + static_cast<size_t>(work - tile * kSplits) * p.M * p.ldc;
 			const float* __restrict__ R = p.residual != nullptr ? p.residual + tc.batch * p.strideC : nullptr;
@@ -1186,6 +1170,7 @@ int launch_bn(const ContractionParams& p0, int batch, cudaStream_t stream)
 			smemBytes = static_cast<size_t>(rawSlots) * slotBytes + fixedBytes;
 		}
 	}
+	p.div = tile_divs(p, nTiles, tilesPerBatch);
 	const int nt = static_cast<int>(numWork), nn = static_cast<int>(nTiles), tpb = static_cast<int>(tilesPerBatch);
 	cudaEvent_t timedStart = nullptr, timedStop = nullptr;
 	const bool timed = timing_events(&timedStart, &timedStop);
@@ -1206,6 +1191,21 @@ int launch_bn(const ContractionParams& p0, int batch, cudaStream_t stream)
 }
 
 } // namespace
+
+FastDiv fast_div(long long d)
+{
+	FastDiv f = {};
+	while((1LL << f.shift) < d) ++f.shift;
+	f.mul = static_cast<uint32_t>(((1ULL << 32) * static_cast<unsigned long long>((1LL << f.shift) - d)) / static_cast<unsigned long long>(d) + 1);
+	return f;
+}
+
+TileDivs tile_divs(const ContractionParams& p, long long nTiles, long long tilesPerBatch)
+{
+	const bool conv = p.a_mode != A_ROWS;
+	return { fast_div(p.kSplits > 1 ? p.kSplits : 1), fast_div(tilesPerBatch), fast_div(nTiles), fast_div(conv ? p.Ho : 1),
+		fast_div(conv ? static_cast<long long>(p.Ho) * p.Wo : 1), fast_div(conv ? p.Wo : 1) };
+}
 
 // Few tiles and a long K loop (small batches: a handful of CTAs would walk dozens of K blocks while the other SMs idle): cut
 // every tile's K loop into equal parts that run as separate work items and store their partial sums in slabs of the
