@@ -154,11 +154,14 @@ size_t prepared_filter_floats(long long k, long long r, long long s, long long c
 // contraction_split.cu) when its second operand is prepared.  From the tile count on that no longer splits K it does so
 // from five K blocks on (a shorter loop is hidden behind its epilogue; ResNet-50 at batch 256, TF32 against fp16 kernel: K =
 // 64 and 128 with residual 355 / 430 us and 197 / 239, K = 256 158 / 150, K = 1152 284 / 195).  With fewer tiles a launch is
-// a few K blocks per part and a finishing pass in either kernel: it does from 32 K blocks on.
+// a few K blocks per part and a finishing pass in either kernel: 4116 rows x 256 columns took 12.9 / 13.0 us at K = 256, 16.0 /
+// 15.0 at 576, 18.1 / 16.2 at 768, 32.8 / 25.5 at 2304, 1029 x 512 13.3 / 14.5 at 384 and 14.8 / 14.0 at 768.  It goes there
+// from 24 K blocks on, where the gain is clear of the spread at every size tried; below, a launch keeps the bits of the
+// kernel that gathers its operands.
 bool split_form_pays(long long mTiles, long long n, long long k, long long batch)
 {
 	const int width = contraction_tile_width(static_cast<int>(n));
-	return k > (mTiles * ((n + width - 1) / width) * batch > SPLIT_TILES_MAX ? 128 : 1023);
+	return k > (mTiles * ((n + width - 1) / width) * batch > SPLIT_TILES_MAX ? 128 : 767);
 }
 
 // Row-window form of a convolution with few channels (the network stem): the image is copied once with its spatial

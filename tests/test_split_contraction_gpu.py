@@ -49,10 +49,10 @@ def rows_of(kind: str, m: int, k: int, g) -> torch.Tensor:
 
 
 # m x k x n: 75 row tiles are the fewest that one column tile takes to this kernel, 160 = five K blocks the shortest depth; the
-# last three have few tiles and split K (into 2, 8 and, with 33 K blocks, 3 parts)
+# last four have few tiles and split K (into 2, 8, with 33 K blocks 3, and 4 parts)
 @pytest.mark.parametrize("m,k,n", [(75 * 128 - 127, 160, 32), (9700, 132, 57), (9600, 190, 64), (9601, 576, 96), (4800, 320, 129),
                                    (1024, 333 * 4, 1300), (5000, 2064, 260), (4116, 1024, 256),
-                                   (1029, 2304, 128), (1100, 1044, 132)])
+                                   (1029, 2304, 128), (1100, 1044, 132), (1024, 768, 512)])
 @pytest.mark.parametrize("kind", ["normal", "zeros", "scales", "rising", "jump"])
 def test_products(ops, m, k, n, kind):
     g = torch.Generator(device="cuda")
