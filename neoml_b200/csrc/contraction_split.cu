@@ -642,7 +642,7 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 // packed[n * numKb * 32 floats], and scales[n] = 1 / s_n.  A row is held in registers between the search for its maximum
 // and the split (up to 8 x 16 bytes per thread; the rest of a longer row is read again): by one warp where that suffices
 // (K <= 1024), four rows to a block, else by the block.  Bound: memory, and for a layer's filter the launch itself.
-// 4096 x 4096: 60 us with two passes of dependent loads, see the launch below for what it takes now.
+// (4096 x 4096 took 60 us as two passes of dependent loads, one quad of a thread after the other.)
 // WINDOW: the row is a convolution filter of r rows x s taps x c channels, and each filter row is widened to 32 floats
 // (tap j / c4, channel j % c4), the row-window form of a few-channel layer.
 struct RowWindow {
