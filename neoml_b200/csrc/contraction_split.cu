@@ -74,6 +74,7 @@ constexpr int MAX_RAW_SLOTS = 8;
 constexpr int SCALE_RING = STAGES + 4;
 constexpr float LO_SCALE = 2048.f;
 constexpr int TARGET_EXP = 9;              // log2 of where a row's first maximum is put
+constexpr int SCALE_EXP_MAX = 254 - 11;    // biased exponent of the largest scale: LO_SCALE (2^11) times it is still finite
 constexpr float RAISE_AT = 32768.f;        // a scaled element beyond this moves the row's scale (fp16 ends at 65504)
 
 enum {
@@ -86,13 +87,14 @@ __device__ __forceinline__ uint32_t swz(int row, int chunk)
 	return static_cast<uint32_t>(row) * 128u + (static_cast<uint32_t>(chunk ^ (row & 7)) << 4);
 }
 
-// The power of two that puts `largest` into [2^TARGET_EXP, 2^(TARGET_EXP + 1)), kept where it and its inverse are
-// normal numbers (an infinite element keeps being infinite, a vanishing one vanishes).
+// The power of two that puts `largest` into [2^TARGET_EXP, 2^(TARGET_EXP + 1)), kept where its inverse and LO_SCALE times it
+// are normal numbers: at most 2^116, which leaves even the smallest normal element at 2^-10 (an infinite element keeps being
+// infinite).  With 2^126 as the limit t = LO_SCALE * s below was infinite from maxima of 2^-107 down, and with it the lo halves.
 __device__ __forceinline__ float scale_for(float largest)
 {
 	const int e = static_cast<int>(__float_as_uint(largest) >> 23) & 0xff;
 	int se = 254 + TARGET_EXP - e;
-	se = se < 1 ? 1 : (se > 253 ? 253 : se);
+	se = se < 1 ? 1 : (se > SCALE_EXP_MAX ? SCALE_EXP_MAX : se);
 	return __uint_as_float(static_cast<uint32_t>(se) << 23);
 }
 // 1 / s of such a power of two
@@ -108,7 +110,7 @@ __device__ __forceinline__ void split_pair(float x0, float x1, float s, float t,
 	float a, b, c, d;
 	asm("{\n\t.reg .b64 x, s, t, a, c;\n\t"
 		"mov.b64 x, {%4, %5};\n\tmov.b64 s, {%6, %6};\n\tmov.b64 t, {%7, %7};\n\t"
-		"mul.rn.ftz.f32x2 a, x, s;\n\tmul.rn.ftz.f32x2 c, x, t;\n\t"
+		"mul.rn.f32x2 a, x, s;\n\tmul.rn.f32x2 c, x, t;\n\t" // subnormal elements count, too
 		"mov.b64 {%0, %1}, a;\n\tmov.b64 {%2, %3}, c;\n\t}"
 		: "=f"(a), "=f"(b), "=f"(c), "=f"(d) : "f"(x0), "f"(x1), "f"(s), "f"(t));
 	const __half2 h = __floats2half2_rn(a, b);

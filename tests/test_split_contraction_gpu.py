@@ -68,6 +68,27 @@ def test_products(ops, m, k, n, kind):
         assert worst(got, a, b, extra=bias + res) < bound(k)
 
 
+@pytest.mark.parametrize("m,k,n", [(9601, 160, 40), (1100, 1044, 132)])
+def test_tiny_rows(ops, m, k, n):
+    """Rows whose first K block, or which altogether, lie at the lower end of fp32; zeros among them."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(m)
+    a, b = torch.empty(m, k, device="cuda").normal_(generator=g), torch.empty(n, k, device="cuda").normal_(generator=g)
+    a[:, :32] *= torch.logspace(-37, -30, m, device="cuda")[:, None]
+    a[:, 1:32:3] = 0
+    first = a[:, :32].clone()
+    a[::7, :32] *= 1e-6       # with the line before: a first block of zeros and subnormal numbers for some
+    b[::3] *= torch.logspace(-33, -29, b[::3].shape[0], device="cuda")[:, None]
+    b[::3, ::4] = 0
+    got = ops.MultiplyMatrixByTransposedMatrix(a, b)
+    assert bool(torch.isfinite(got).all()) and worst(got, a, b) < bound(k)
+    a[::2, 32:] = 0           # nothing but the tiny block
+    a[:, :32] = first
+    b[::3] = torch.empty(b[::3].shape, device="cuda").normal_(generator=g) * 1e33
+    got = ops.MultiplyMatrixByTransposedMatrix(a, b)
+    assert bool(torch.isfinite(got).all()) and worst(got[:, ::3], a, b[::3]) < bound(k)
+
+
 def test_batches_and_infinities(ops):
     g = torch.Generator(device="cuda")
     g.manual_seed(5)
