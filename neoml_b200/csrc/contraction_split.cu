@@ -103,6 +103,18 @@ __device__ __forceinline__ float inverse_scale(float s)
 	return __uint_as_float((254u << 23) - __float_as_uint(s));
 }
 
+// v * rowInv * colInv for powers of two whose product with v may leave fp32's range although all three together do not (rows of
+// 1e34 by columns of 1e-30): the exponents are added and applied in two halves of one sign, so that a step overflows or
+// vanishes only where the result does.
+__device__ __forceinline__ float unscale(float v, float rowInv, float colInv)
+{
+	const int e = static_cast<int>(__float_as_uint(rowInv) >> 23) + static_cast<int>(__float_as_uint(colInv) >> 23) - 254;
+	const int half = e >> 1;
+	return v * __uint_as_float(static_cast<uint32_t>(127 + half) << 23) * __uint_as_float(static_cast<uint32_t>(127 + e - half) << 23);
+}
+// The accumulators stay below 2^50 or so and sums of any weight above 2^-40: within these limits v * rowInv is safe by itself.
+constexpr float ROW_INV_MIN = 0x1p-64f, ROW_INV_MAX = 0x1p64f;
+
 // hi and lo halves of two scaled neighbours, the first in the low half; t = LO_SCALE * s.  (x0, x1) as packed pairs: the
 // converters are bound by instruction issue.
 __device__ __forceinline__ void split_pair(float x0, float x1, float s, float t, uint32_t& hi, uint32_t& lo)
@@ -511,8 +523,35 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 				__syncwarp();
 				if(lane == 0) mbar_arrive(crossEmptyBar);
 			}
-			const float inv = rowInv[ring * BM + quad * 32 + lane];
+			float inv = rowInv[ring * BM + quad * 32 + lane];
 			if(++ring == SCALE_RING) ring = 0;
+			// Where the row's scale alone might take a sum out of range, both scales are applied at once, ahead of the loop below:
+			// rare, and a branch per warp and tile.
+			const bool careful = __any_sync(0xffffffffu, inv < ROW_INV_MIN || inv > ROW_INV_MAX) != 0;
+			if(careful) {
+#pragma unroll 1
+				for(int g = 0; g < HALF_COLS; g += 16) {
+					uint32_t a[16];
+					tmem_ld16_issue(accMain + g, a);
+					if(!FOLD) {
+						uint32_t b[16];
+						tmem_ld16_issue(accCross + g, b);
+						tmem_ld_wait();
+#pragma unroll
+						for(int i = 0; i < 16; ++i) {
+							a[i] = __float_as_uint(fmaf(__uint_as_float(b[i]), 1.f / LO_SCALE, __uint_as_float(a[i])));
+							b[i] = 0u;
+						}
+						tmem_st16(accCross + g, b);
+					}
+					tmem_ld_wait();
+#pragma unroll
+					for(int i = 0; i < 16; ++i) a[i] = __float_as_uint(unscale(__uint_as_float(a[i]), inv, scaleStrip[g + i]));
+					tmem_st16(accMain + g, a);
+				}
+				tmem_st_wait();
+				inv = 1.f;
+			}
 
 			float4 res[4], resNext[4];
 			if(useRes) load_res(0, res);
@@ -550,7 +589,8 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 				}
 				__syncwarp();
 				const float4 bias4 = *reinterpret_cast<const float4*>(biasStrip + ch * 16 + c4 * 4);
-				const float4 scale4 = *reinterpret_cast<const float4*>(scaleStrip + ch * 16 + c4 * 4);
+				float4 scale4 = make_float4(1.f, 1.f, 1.f, 1.f);
+				if(!careful) scale4 = *reinterpret_cast<const float4*>(scaleStrip + ch * 16 + c4 * 4);
 				float4 ov[4];
 #pragma unroll
 				for(int i = 0; i < 4; ++i) {

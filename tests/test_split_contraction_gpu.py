@@ -89,6 +89,22 @@ def test_tiny_rows(ops, m, k, n):
     assert bool(torch.isfinite(got).all()) and worst(got[:, ::3], a, b[::3]) < bound(k)
 
 
+@pytest.mark.parametrize("m,k,n", [(9601, 160, 40), (4800, 192, 129), (1100, 1044, 132)])
+def test_both_scales_over_the_whole_range(ops, m, k, n):
+    """Rows of every magnitude by columns of every magnitude: a result is finite and right wherever fp32 holds it."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(m)
+    a, b = torch.empty(m, k, device="cuda").normal_(generator=g), torch.empty(n, k, device="cuda").normal_(generator=g)
+    a *= torch.logspace(-32, 36, m, device="cuda")[:, None]
+    b *= torch.logspace(-32, 36, n, device="cuda")[:, None]
+    got = ops.MultiplyMatrixByTransposedMatrix(a, b)
+    size = a.abs().double() @ b.abs().double().T
+    held = (size > 1e-30) & (size < 3e38)
+    assert float(held.double().mean()) > 0.7 and bool(torch.isfinite(got[held]).all())
+    err = (got.double() - a.double() @ b.double().T).abs() / size
+    assert float(err[held].max()) < bound(k)
+
+
 def test_batches_and_infinities(ops):
     g = torch.Generator(device="cuda")
     g.manual_seed(5)
