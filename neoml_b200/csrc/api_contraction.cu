@@ -157,11 +157,12 @@ size_t prepared_filter_floats(long long k, long long r, long long s, long long c
 // a few K blocks per part and a finishing pass in either kernel: 4116 rows x 256 columns took 12.9 / 13.0 us at K = 256, 16.0 /
 // 15.0 at 576, 18.1 / 16.2 at 768, 32.8 / 25.5 at 2304, 1029 x 512 13.3 / 14.5 at 384 and 14.8 / 14.0 at 768.  It goes there
 // from 24 K blocks on, where the gain is clear of the spread at every size tried; below, a launch keeps the bits of the
-// kernel that gathers its operands.
+// kernel that gathers its operands.  Deeper products than 2^18 stay on the TF32 kernel: a tile of them whose sums all had to be
+// formed anew (contraction_split.cu, small_sums) would come near the two seconds after which a wait gives up.
 bool split_form_pays(long long mTiles, long long n, long long k, long long batch)
 {
 	const int width = contraction_tile_width(static_cast<int>(n));
-	return k > (mTiles * ((n + width - 1) / width) * batch > SPLIT_TILES_MAX ? 128 : 767);
+	return k > (mTiles * ((n + width - 1) / width) * batch > SPLIT_TILES_MAX ? 128 : 767) && k <= (1 << 18);
 }
 
 // Row-window form of a convolution with few channels (the network stem): the image is copied once with its spatial
@@ -626,7 +627,10 @@ int blob_convolution(void* stream, const nb200_conv_desc* d, const float* x, con
 		p.A = xs; p.B = split ? filter : precision == NB200_PREC_3XTF32 ? fs : fprep; p.C = y;
 		p.Blo = precision == NB200_PREC_3XTF32 && !split ? fprep : nullptr;
 		p.b_ready = 1;
-		if(split) set_split_operand(p, fsplit, d->k, d->r * 32LL);
+		if(split) {
+			set_split_operand(p, fsplit, d->k, d->r * 32LL);
+			p.filterS = d->s; p.filterC = d->c;
+		}
 		p.M = d->batch * d->ho * d->wo; p.N = d->k; p.K = d->r * 32;
 		p.lda = 0; p.ldb = p.K; p.ldc = d->k;
 		p.a_mode = A_CONV_WINDOW; p.b_mode = B_ROWS; p.a_vec = 1; p.b_vec = 1;

@@ -53,7 +53,8 @@ struct ContractionParams {
 	                  // and for plain TF32 a pre-rounded B passed as B itself, the kernel does no per-step work on B
 	const float* bSplit; // optional (3xTF32, all-TMA first operand): B in the split form of split_operand(); the launch then goes
 	                     // to the fp16 kernel of contraction_split.cu
-	const float* bScale; // with bSplit: 1 / s_n of its rows, batch entries one after another
+	const float* bScale; // with bSplit: 1 / s_n of its rows, batch entries one after another; B stays the operand as it is
+	int filterS, filterC; // with bSplit and A_CONV_WINDOW: columns and channels of the filter in B
 	int kSplits;      // > 1: every tile's K loop is cut into this many equal parts that run as separate work items (few-tile
 	                  // launches: latency at small batch).  Part i stores its partial result at C + i * M * ldc, where C
 	                  // is then the caller's split scratch; a finishing pass sums the parts in order (deterministic) and

@@ -17,10 +17,18 @@
 // its largest element between 2^9 and 2^10; from there elements may grow 2^5-fold at least before the scale has to
 // change.  When a later block does exceed that, the converter warp waits for the products issued so far and divides its
 // rows of the accumulators by the (power of two) change of scale before it goes on: exact, rare on ordinary data, right
-// on any.  Small elements: an element is held to 22 bits or to 2^-36 in scaled units, whichever is coarser, that is to
-// 2^-45 of the first block's maximum (A) and 2^-50 of its row's maximum (B).  An element more than 2^23 below its row's
-// maximum therefore loses bits that the three TF32 products keep; it takes weights as far apart the other way for that
-// to reach the result (a row of 1e6 and 1e-6 times weights of 1e-6 and 1e6: 1e-4).
+// on any.
+// Small elements: from 2^-14 up in scaled units an element keeps its 22 bits; below, it is held to 2^-36, and both operands'
+// together put an error of at most 2^-20 on each of a result's products (the other factor is below 2^15).  With
+// S = sum |a||b| in scaled units, K * 2^-20 <= K * 2^-25 * S wherever S >= 2^5, as much as the accumulation of three TF32
+// products may take.  S >= 2^5 follows from a sum of 2^5 or more, and from a main part of 2^5 + K * 2^-8 or more (an element's hi half
+// is larger than the element by 2^-11 of it or by 2^-25 at most).  The sums of which neither holds -- of ordinary operands
+// one in 10^8 -- the epilogue looks into (small_sums): where the row of A or the row of B holds such elements the sum is
+// formed anew from the fp32 operands.  That serves rows whose large elements meet small or no ones on the other side
+// (1e6 and 1e-6 by weights of 1e-6 and 1e6: 5e-3 of sum |a||b| without it); a launch of nothing but such sums takes some 15
+// times as long.  The look at every sum costs 1 to 4 % of an ordinary launch; marks of A's rows from the converters, which
+// every block would pay for, cost 10 to 18 %.
+// A row of subnormal numbers alone counts where its first K block holds one.
 //
 // Pipeline: as in contraction_tc.cu, a persistent CTA per SM (24 warps) walks the 128 x BN tiles:
 //   warps 0, 1   copy by TMA into a ring of raw slots: A (128 rows x 32 floats; plain rows, im2col or row windows) and B
@@ -75,6 +83,8 @@ constexpr int SCALE_RING = STAGES + 4;
 constexpr float LO_SCALE = 2048.f;
 constexpr int TARGET_EXP = 9;              // log2 of where a row's first maximum is put
 constexpr int SCALE_EXP_MAX = 254 - 11;    // biased exponent of the largest scale: LO_SCALE (2^11) times it is still finite
+constexpr float FULL_BITS = 0x1p-14f;      // a scaled element below this has fewer than 22 bits
+constexpr float SMALL_SUM = 32.f;          // see Range: sums that are smaller (scaled), and their main parts, are looked into
 constexpr float RAISE_AT = 32768.f;        // a scaled element beyond this moves the row's scale (fp16 ends at 65504)
 
 enum {
@@ -101,6 +111,21 @@ __device__ __forceinline__ float scale_for(float largest)
 __device__ __forceinline__ float inverse_scale(float s)
 {
 	return __uint_as_float((254u << 23) - __float_as_uint(s));
+}
+
+// Order-preserving key of |x|, zero last: the smallest key of a set is its smallest element that is not zero.
+__device__ __forceinline__ uint32_t small_key(float x)
+{
+	return 2u * __float_as_uint(x) - 1u;
+}
+// The key below which the elements of a row with this inverse scale have fewer than 22 bits (subnormal ones among them).
+__device__ __forceinline__ uint32_t coarse_below(float inv)
+{
+	return small_key(fmaxf(FULL_BITS * inv, 0x1p-126f));
+}
+__device__ __forceinline__ uint32_t smallest_key(uint32_t m, const float4& v)
+{
+	return min(min(min(m, small_key(v.x)), min(small_key(v.y), small_key(v.z))), small_key(v.w));
 }
 
 // v * rowInv * colInv for powers of two whose product with v may leave fp32's range although all three together do not (rows of
@@ -145,6 +170,92 @@ __device__ __forceinline__ float max_abs(float m, const float4& v)
 	return r;
 }
 
+__device__ __forceinline__ float min3(float a, float b, float c)
+{
+	asm("min.ftz.f32 %0, %0, %1, %2;" : "+f"(a) : "f"(b), "f"(c));
+	return a;
+}
+
+// The 32 floats of K block kb in row m of the first operand (`at`: conv_row of m), or null where they are a convolution's padding.
+__device__ __forceinline__ const float* row_block(const ContractionParams& p, const float* A, const ConvRow& at, int m, int kb)
+{
+	if(p.a_mode == A_ROWS) return A + static_cast<size_t>(m) * p.lda + kb * BK;
+	int iy = at.iy0 + kb, ix = at.ix0, c = 0; // windows: a block per image row, the padding is in the copy
+	if(p.a_mode == A_CONV_TAP) {
+		const int tap = kb * BK / p.Cin, fr = tap / p.S;
+		c = kb * BK - tap * p.Cin;
+		iy = at.iy0 + fr * p.dilH;
+		ix = at.ix0 + (tap - fr * p.S) * p.dilW;
+		if(static_cast<unsigned>(iy) >= static_cast<unsigned>(p.H) || static_cast<unsigned>(ix) >= static_cast<unsigned>(p.W)) return nullptr;
+	}
+	return A + at.base + (iy * p.W + ix) * p.Cin + c;
+}
+
+// The sums that came out small.  A warp's lane r has the bits of those among the 16 columns from n0 on that belong to row m0 + r;
+// their finished values lie in its 64 bytes of the staging slice.  A row of A is looked through for elements of fewer than
+// 22 bits while its first four columns are formed (`clean`: the rows that have none), rows of B carry the mark in their
+// scale (`markedCols`); a sum with such elements on either side is formed anew: fused multiply-adds of the fp32 operands, 32
+// partial sums along K, subnormal numbers included.  Four columns at a time, as whole tiles of such sums occur in data that
+// is made for it.
+__device__ __forceinline__ void small_sums(const ContractionParams& p, uint32_t small, uint32_t markedCols, float inv, int batch, int m0,
+	int n0, int kbBegin, int kbEnd, uint8_t* stg, uint32_t& clean)
+{
+	const int lane = threadIdx.x & 31;
+	const float* A = p.A + batch * p.strideA;
+	const float* B = p.B + batch * p.strideB;
+#pragma unroll 1
+	for(uint32_t rows = __ballot_sync(0xffffffffu, small != 0); rows != 0; rows &= rows - 1) {
+		const int r = __ffs(rows) - 1, m = m0 + r;
+		uint32_t cols = __shfl_sync(0xffffffffu, small, r);
+		if(clean >> r & 1u) cols &= markedCols;
+		const uint32_t below = coarse_below(__shfl_sync(0xffffffffu, inv, r));
+		const ConvRow at = p.a_mode == A_ROWS ? ConvRow{} : conv_row(p, m);
+#pragma unroll 1
+		while(cols != 0) {
+			const int q = (__ffs(cols) - 1) >> 2;
+			float sum[4] = { 0.f, 0.f, 0.f, 0.f };
+			uint32_t smallest = 0xffffffffu;
+#pragma unroll 1
+			for(int kb = kbBegin; kb < kbEnd; ++kb) {
+				const float* src = row_block(p, A, at, m, kb);
+				bool real = src != nullptr && kb * BK + lane < p.K;
+				int b = kb * BK + lane;
+				long long step = p.ldb;
+				if(p.a_mode == A_CONV_WINDOW) {
+					// the filter as the caller has it: channels and taps that are not there count nothing
+					const int tap = lane / p.Cin, ch = lane - tap * p.Cin;
+					real = tap < p.filterS && ch < p.filterC;
+					b = (kb * p.filterS + tap) * p.filterC + ch;
+					step = static_cast<long long>(p.K / BK) * p.filterS * p.filterC;
+				}
+				if(real) {
+					const float a = __ldg(src + lane);
+					smallest = min(smallest, small_key(a));
+#pragma unroll
+					for(int t = 0; t < 4; ++t) {
+						const float w = __ldg(B + min(n0 + 4 * q + t, p.N - 1) * step + b);
+						asm("fma.rn.f32 %0, %1, %2, %0;" : "+f"(sum[t]) : "f"(a), "f"(w));
+					}
+				}
+			}
+			if(!__any_sync(0xffffffffu, smallest < below)) {
+				clean |= 1u << r;
+				cols &= markedCols;
+			}
+			float mine = 0.f; // of column 4 q + lane
+#pragma unroll
+			for(int t = 0; t < 4; ++t) {
+#pragma unroll
+				for(int o = 16; o > 0; o >>= 1) sum[t] += __shfl_xor_sync(0xffffffffu, sum[t], o);
+				if(lane == t) mine = sum[t];
+			}
+			const uint32_t four = (cols >> (4 * q)) & 15u;
+			if((four >> lane) & 1u) reinterpret_cast<float*>(stg + r * 64)[4 * q + lane] = mine;
+			cols &= ~(15u << (4 * q));
+		}
+	}
+}
+
 template<int BN>
 __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const ContractionParams p, int numTiles, int nTiles,
 	int tilesPerBatch, int rawSlots, const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB)
@@ -155,8 +266,8 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 
 	constexpr int B_TILE_BYTES = BN * B_ROW_BYTES;
 	// Two main accumulators (the epilogue of tile i overlaps the products of tile i + 1) and as many cross accumulators
-	// as fit beside the stages; where that is one (BN = 128) the epilogue first folds it into the main accumulator in
-	// place and hands it back.
+	// as fit beside the stages; the epilogue first folds a tile's into its main accumulator, and where there is but one
+	// (BN = 128) hands it back.
 	constexpr bool FOLD = BN > 96;
 	constexpr uint32_t CROSS_BASE = 2 * BN;
 	constexpr uint32_t A_BASE = (FOLD ? 3 : 4) * BN;
@@ -173,8 +284,8 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 
 	uint8_t* rawRing = smem;
 	uint8_t* staging = rawRing + static_cast<size_t>(rawSlots) * SLOT_BYTES;
-	float* strips = reinterpret_cast<float*>(staging + EPI_WARPS * STAGING_BYTES_PER_WARP); // per warp: bias, column scale
-	float* rowInv = strips + EPI_WARPS * 2 * HALF_COLS;
+	float* strips = reinterpret_cast<float*>(staging + EPI_WARPS * STAGING_BYTES_PER_WARP); // per warp: bias, column scale, large for columns that are not there or zero
+	float* rowInv = strips + EPI_WARPS * 3 * HALF_COLS;
 	float* rowScale = rowInv + SCALE_RING * BM; // the scale of each row of the tile being converted
 	uint64_t* rawFullBar = reinterpret_cast<uint64_t*>(rowScale + BM);
 	uint64_t* rawEmptyBar = rawFullBar + MAX_RAW_SLOTS;
@@ -373,8 +484,18 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 			// the scale after the K block before, which the group before has looked at
 			if(step > 0 && !mbar_wait_bounded_warp(chainBefore, (group > 0 ? n : n - 1) & 1, abortFlag, p.status, SITE_CHAIN)) break;
 			float s = kb > 0 ? rowScale[row] : 0.f; // 0: nothing but zeros so far
-			const bool move = s == 0.f ? largest > 0.f : largest * s > RAISE_AT;
+			bool move = s == 0.f ? largest > 0.f : largest * s > RAISE_AT;
 			if(kb == 0 || __any_sync(0xffffffffu, move)) {
+				// of a row that holds zeros or subnormal numbers, which max_abs takes for zeros, the latter count as the smallest
+				// normal number (no branch: its code would be fetched anew by every launch)
+				uint32_t bits = 0;
+#pragma unroll
+				for(int c = 0; c < 8; ++c) {
+					bits |= __float_as_uint(x[c].x) | __float_as_uint(x[c].y) | __float_as_uint(x[c].z) | __float_as_uint(x[c].w);
+				}
+				const bool subnormal = s == 0.f && largest == 0.f && (bits << 1) != 0;
+				largest = subnormal ? 0x1p-126f : largest;
+				move = move || subnormal;
 				const float next = move ? scale_for(largest) : s;
 				if(__any_sync(0xffffffffu, move && s != 0.f)) {
 					// rare: rows whose accumulated sums are in the old scale.  The products issued so far must have
@@ -417,7 +538,7 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 				tmem_st16(laneBase + A_BASE + group * STAGE_COLS + 16 * half, r);
 			}
 			const bool last = kb == numKb - 1;
-			if(last) rowInv[ring * BM + row] = s == 0.f ? 1.f : inverse_scale(s);
+			if(last) rowInv[ring * BM + row] = s == 0.f ? 0.f : inverse_scale(s); // 0: a row of zeros
 			slot += CVT_GROUPS;
 			while(slot >= rawSlots) { slot -= rawSlots; rawParity ^= 1; }
 			tmem_st_wait();
@@ -444,8 +565,9 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 		const int rowInGroup = lane >> 2;  // 0..7: which of the 8 rows a warp-wide 16-byte access covers
 		const int c4 = lane & 3;           // which 16-byte piece of the 64-byte row slice
 		const bool vec = p.c_vec != 0;
-		float* biasStrip = strips + ew * 2 * HALF_COLS;
+		float* biasStrip = strips + ew * 3 * HALF_COLS;
 		float* scaleStrip = biasStrip + HALF_COLS;
+		float* skipStrip = scaleStrip + HALF_COLS;
 		int stripCol = -1, stripBatch = -1;
 		const bool fastStore = vec && p.accumulate == 0 && p.act != NB200_ACT_HSWISH && p.act != NB200_ACT_SIGMOID_GATE;
 		const bool gateStore = vec && p.accumulate == 0 && p.act == NB200_ACT_SIGMOID_GATE;
@@ -453,6 +575,7 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 		const bool clampOn = p.act == NB200_ACT_RELU;
 		const float actParam = p.act_param_device != nullptr ? __ldg(p.act_param_device) : p.act_param;
 		const float clampHi = actParam > 0.f ? actParam : __int_as_float(0x7f800000);
+		const float small = 2.f * (SMALL_SUM + numKb * (BK / 256.f));
 		bool ok = true;
 		int ring = 0;
 		for(int local = 0; local < myTiles && ok; ++local) {
@@ -485,7 +608,9 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 				for(int j = lane; j < HALF_COLS; j += 32) {
 					const int n = colBase + j;
 					biasStrip[j] = (p.bias != nullptr && n < p.N) ? __ldg(p.bias + n) : 0.f;
-					scaleStrip[j] = n < p.N ? __ldg(p.bScale + static_cast<size_t>(tc.batch) * p.N + n) : 0.f;
+					const float scale = n < p.N ? __ldg(p.bScale + static_cast<size_t>(tc.batch) * p.N + n) : 0.f;
+					scaleStrip[j] = scale;
+					skipStrip[j] = scale == 0.f ? 1e30f : 0.f;
 				}
 				stripCol = colBase;
 				stripBatch = tc.batch;
@@ -507,46 +632,66 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 			const uint32_t laneCol = (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(half * HALF_COLS);
 			const uint32_t accMain = tmemBase + set * BN + laneCol;
 			const uint32_t accCross = tmemBase + CROSS_BASE + (FOLD ? 0 : set * BN) + laneCol;
-			if(FOLD) {
+			// The cross terms are folded into the main accumulator in place, with a look at how small the sums are (not unrolled: with
+			// that the 128-column kernel spilled, a 28 x 28, 512 -> 128 layer at batch 21 took 13.4 us for 12.8).
+			float inv = rowInv[ring * BM + quad * 32 + lane];
+			const bool alive = inv != 0.f && rowBase + lane < mEnd; // a row that exists and is not all zeros
+			float least = __int_as_float(0x7f800000);
+#pragma unroll 1
+			for(int g = 0; g < HALF_COLS; g += 16) {
+				uint32_t a[16], b[16];
+				tmem_ld16_issue(accMain + g, a);
+				tmem_ld16_issue(accCross + g, b);
+				tmem_ld_wait();
 #pragma unroll
-				for(int g = 0; g < HALF_COLS; g += 16) {
-					uint32_t a[16], b[16];
-					tmem_ld16_issue(accMain + g, a);
-					tmem_ld16_issue(accCross + g, b);
-					tmem_ld_wait();
-#pragma unroll
-					for(int i = 0; i < 16; ++i) a[i] = __float_as_uint(fmaf(__uint_as_float(b[i]), 1.f / LO_SCALE, __uint_as_float(a[i])));
-					tmem_st16(accMain + g, a);
+				for(int i = 0; i < 16; i += 2) {
+					const float x = __uint_as_float(a[i]), y = __uint_as_float(a[i + 1]);
+					const float v = fmaf(__uint_as_float(b[i]), 1.f / LO_SCALE, x), w = fmaf(__uint_as_float(b[i + 1]), 1.f / LO_SCALE, y);
+					const float2 skip = *reinterpret_cast<const float2*>(skipStrip + g + i);
+					least = min3(least, fabsf(v) + (fabsf(x) + skip.x), fabsf(w) + (fabsf(y) + skip.y));
+					a[i] = __float_as_uint(v);
+					a[i + 1] = __float_as_uint(w);
 				}
-				tmem_st_wait();
+				tmem_st16(accMain + g, a);
+			}
+			tmem_st_wait();
+			if(FOLD) {
 				tc_fence_before_sync();
 				__syncwarp();
 				if(lane == 0) mbar_arrive(crossEmptyBar);
 			}
-			float inv = rowInv[ring * BM + quad * 32 + lane];
 			if(++ring == SCALE_RING) ring = 0;
-			// Where the row's scale alone might take a sum out of range, both scales are applied at once, ahead of the loop below:
-			// rare, and a branch per warp and tile.
-			const bool careful = __any_sync(0xffffffffu, inv < ROW_INV_MIN || inv > ROW_INV_MAX) != 0;
-			if(careful) {
+			// Where the row's scale alone might take a sum out of range both scales are applied at once, and small sums are looked
+			// into, ahead of the loop below: rare, and a branch per warp and tile.
+			const bool careful = __any_sync(0xffffffffu, (alive && least < small) || (inv < ROW_INV_MIN && inv != 0.f) || inv > ROW_INV_MAX) != 0;
+			if(__builtin_expect(careful, 0)) {
+				uint32_t clean = 0;
+				float* mine = reinterpret_cast<float*>(stg + lane * 64);
 #pragma unroll 1
 				for(int g = 0; g < HALF_COLS; g += 16) {
-					uint32_t a[16];
+					uint32_t a[16], smallCols = 0, markedCols = 0;
 					tmem_ld16_issue(accMain + g, a);
-					if(!FOLD) {
-						uint32_t b[16];
-						tmem_ld16_issue(accCross + g, b);
-						tmem_ld_wait();
-#pragma unroll
-						for(int i = 0; i < 16; ++i) {
-							a[i] = __float_as_uint(fmaf(__uint_as_float(b[i]), 1.f / LO_SCALE, __uint_as_float(a[i])));
-							b[i] = 0u;
-						}
-						tmem_st16(accCross + g, b);
-					}
 					tmem_ld_wait();
 #pragma unroll
-					for(int i = 0; i < 16; ++i) a[i] = __float_as_uint(unscale(__uint_as_float(a[i]), inv, scaleStrip[g + i]));
+					for(int q = 0; q < 4; ++q) reinterpret_cast<uint4*>(mine)[q] = make_uint4(a[4 * q], a[4 * q + 1], a[4 * q + 2], a[4 * q + 3]);
+#pragma unroll 1
+					for(int i = 0; i < 16; ++i) {
+						const float v = mine[i], scale = scaleStrip[g + i]; // 0: a row of B that is all zeros, or none
+						// (rows this tiny may have lost subnormal elements in blocks before the scale was set)
+						if(alive && scale != 0.f && (fabsf(v) < small || inv < 0x1p-90f)) smallCols |= 1u << i;
+						if(scale < 0.f) markedCols |= 1u << i;
+						mine[i] = unscale(v, inv, fabsf(scale));
+					}
+					__syncwarp();
+					const int kbBegin = (work - tileIdx * kSplits) * numKb;
+					small_sums(p, smallCols, markedCols, inv, tc.batch, rowBase, colBase + g, kbBegin, kbBegin + numKb, stg, clean);
+					__syncwarp();
+#pragma unroll
+					for(int q = 0; q < 4; ++q) {
+						const uint4 o = reinterpret_cast<const uint4*>(mine)[q];
+						a[4 * q] = o.x; a[4 * q + 1] = o.y; a[4 * q + 2] = o.z; a[4 * q + 3] = o.w;
+					}
+					__syncwarp();
 					tmem_st16(accMain + g, a);
 				}
 				tmem_st_wait();
@@ -556,19 +701,14 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 			float4 res[4], resNext[4];
 			if(useRes) load_res(0, res);
 			// 16 columns at a time; the tensor-memory loads of chunk ch + 1 run while chunk ch is transposed and stored
-			uint32_t vm[16], vx[16];
+			uint32_t vm[16];
 			tmem_ld16_issue(accMain, vm);
-			if(!FOLD) tmem_ld16_issue(accCross, vx);
 #pragma unroll
 			for(int ch = 0; ch < CHUNKS; ++ch) {
 				tmem_ld_wait();
 				float v[16];
 #pragma unroll
-				for(int i = 0; i < 16; ++i) {
-					v[i] = __uint_as_float(vm[i]);
-					if(!FOLD) v[i] = fmaf(__uint_as_float(vx[i]), 1.f / LO_SCALE, v[i]);
-					v[i] *= inv;
-				}
+				for(int i = 0; i < 16; ++i) v[i] = __uint_as_float(vm[i]) * inv;
 				const int n = colBase + ch * 16 + c4 * 4; // first of this lane's four columns in the transposed phase
 				const bool colsFull = n + 4 <= p.N;
 				if(useRes && ch + 1 < CHUNKS) load_res(ch + 1, resNext);
@@ -580,7 +720,6 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 				}
 				if(ch + 1 < CHUNKS) {
 					tmem_ld16_issue(accMain + (ch + 1) * 16, vm);
-					if(!FOLD) tmem_ld16_issue(accCross + (ch + 1) * 16, vx);
 				} else {
 					// last read of this tile's accumulators: hand them back
 					tc_fence_before_sync();
@@ -590,7 +729,10 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 				__syncwarp();
 				const float4 bias4 = *reinterpret_cast<const float4*>(biasStrip + ch * 16 + c4 * 4);
 				float4 scale4 = make_float4(1.f, 1.f, 1.f, 1.f);
-				if(!careful) scale4 = *reinterpret_cast<const float4*>(scaleStrip + ch * 16 + c4 * 4);
+				if(!careful) {
+					scale4 = *reinterpret_cast<const float4*>(scaleStrip + ch * 16 + c4 * 4);
+					scale4 = make_float4(fabsf(scale4.x), fabsf(scale4.y), fabsf(scale4.z), fabsf(scale4.w)); // the sign is a mark
+				}
 				float4 ov[4];
 #pragma unroll
 				for(int i = 0; i < 4; ++i) {
@@ -681,7 +823,8 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 }
 
 // B in split form: row n of `rows` becomes numKb blocks of 128 bytes (32 hi halves, 32 lo halves; zeros beyond K) at
-// packed[n * numKb * 32 floats], and scales[n] = 1 / s_n.  A row is held in registers between the search for its maximum
+// packed[n * numKb * 32 floats], and scales[n] = 1 / s_n, negative where the row has elements of fewer than 22 bits, 0 where it
+// has nothing but zeros.  A row is held in registers between the search for its maximum
 // and the split (up to 8 x 16 bytes per thread; the rest of a longer row is read again): by one warp where that suffices
 // (K <= 1024), four rows to a block, else by the block.  Bound: memory, and for a layer's filter the launch itself.
 // (4096 x 4096 took 60 us as two passes of dependent loads, one quad of a thread after the other.)
@@ -701,6 +844,7 @@ __global__ void __launch_bounds__(ROW_THREADS) split_rows_kernel(const float* __
 	dependents_may_start();
 	constexpr int LANES = WARP_ROW ? 32 : ROW_THREADS;
 	__shared__ float warpMax[ROW_THREADS / 32];
+	__shared__ uint32_t warpMin[ROW_THREADS / 32];
 	const int lane = WARP_ROW ? threadIdx.x & 31 : threadIdx.x;
 	const long long row = WARP_ROW ? static_cast<long long>(blockIdx.x) * (ROW_THREADS / 32) + (threadIdx.x >> 5) : blockIdx.x;
 	if(row >= rows) return; // whole warps (WARP_ROW) or none
@@ -729,24 +873,38 @@ __global__ void __launch_bounds__(ROW_THREADS) split_rows_kernel(const float* __
 	const int quads = numKb * 8;
 	float4 held[ROW_QUADS];
 	float largest = 0.f;
+	uint32_t smallest = 0xffffffffu;
 #pragma unroll
 	for(int i = 0; i < ROW_QUADS; ++i) {
 		const int q = lane + i * LANES;
 		held[i] = q < quads ? quad_at(q) : make_float4(0.f, 0.f, 0.f, 0.f);
 	}
 #pragma unroll
-	for(int i = 0; i < ROW_QUADS; ++i) largest = max_abs(largest, held[i]);
-	for(int q = lane + ROW_QUADS * LANES; q < quads; q += LANES) largest = max_abs(largest, quad_at(q));
+	for(int i = 0; i < ROW_QUADS; ++i) {
+		largest = max_abs(largest, held[i]);
+		smallest = smallest_key(smallest, held[i]);
+	}
+	for(int q = lane + ROW_QUADS * LANES; q < quads; q += LANES) {
+		const float4 v = quad_at(q);
+		largest = max_abs(largest, v);
+		smallest = smallest_key(smallest, v);
+	}
 #pragma unroll
 	for(int o = 16; o > 0; o >>= 1) largest = fmaxf(largest, __shfl_xor_sync(0xffffffffu, largest, o));
+	smallest = __reduce_min_sync(0xffffffffu, smallest);
 	if(!WARP_ROW) {
-		if((threadIdx.x & 31) == 0) warpMax[threadIdx.x >> 5] = largest;
+		if((threadIdx.x & 31) == 0) {
+			warpMax[threadIdx.x >> 5] = largest;
+			warpMin[threadIdx.x >> 5] = smallest;
+		}
 		__syncthreads();
 		largest = fmaxf(fmaxf(warpMax[0], warpMax[1]), fmaxf(warpMax[2], warpMax[3]));
+		smallest = min(min(warpMin[0], warpMin[1]), min(warpMin[2], warpMin[3]));
 	}
-	// 2^5 times the target of A's rows: nothing larger follows, so the whole range is used
-	const float s = largest > 0.f ? scale_for(largest * (1.f / 32.f)) : 1.f;
-	if(lane == 0) scales[row] = inverse_scale(s);
+	// 2^5 times the target of A's rows: nothing larger follows, so the whole range is used (subnormal maxima: the largest scale)
+	const bool zeros = smallest == 0xffffffffu;
+	const float s = zeros ? 1.f : scale_for(largest * (1.f / 32.f)), inv = inverse_scale(s);
+	if(lane == 0) scales[row] = zeros ? 0.f : (smallest < coarse_below(inv) ? -inv : inv);
 	uint2* out = packed + row * numKb * 16;
 	auto put = [&](int q, const float4& v) {
 		uint2 hi, lo;
@@ -815,7 +973,7 @@ int launch_bn(const ContractionParams& p0, int batch, cudaStream_t stream)
 	const long long numWork = numTiles * p.kSplits;
 	const int grid = numWork < sms ? static_cast<int>(numWork) : sms;
 	// as many raw slots as fit the 227 KB a CTA may use: the copies run that many K blocks ahead
-	constexpr int fixedBytes = EPI_WARPS * STAGING_BYTES_PER_WARP + EPI_WARPS * BN * 4 /*strips*/ + (SCALE_RING + 1) * BM * 4
+	constexpr int fixedBytes = EPI_WARPS * STAGING_BYTES_PER_WARP + EPI_WARPS * BN * 6 /*strips*/ + (SCALE_RING + 1) * BM * 4
 		+ 512 /*barriers*/ + 1024 /*alignment slack*/;
 	constexpr int slotBytes = A_TILE_BYTES + BN * B_ROW_BYTES;
 	constexpr int fitting = (227 * 1024 - fixedBytes) / slotBytes;

@@ -38,7 +38,7 @@ def rows_of(kind: str, m: int, k: int, g) -> torch.Tensor:
         a.clamp_(min=0)
         a[::2, : k // 2] = 0
         a[::5] = 0
-    elif kind == "scales":       # every row of another magnitude, over fp32's range
+    elif kind == "scales":       # every row of another magnitude
         a *= torch.logspace(-30, 30, m, device="cuda")[:, None]
     elif kind == "rising":       # every K block beyond the range of the one before: the row scales move in mid-tile
         a *= torch.pow(2.0, 7.0 * (torch.arange(k, device="cuda") // 32).clamp(max=12))
@@ -103,6 +103,58 @@ def test_both_scales_over_the_whole_range(ops, m, k, n):
     assert float(held.double().mean()) > 0.7 and bool(torch.isfinite(got[held]).all())
     err = (got.double() - a.double() @ b.double().T).abs() / size
     assert float(err[held].max()) < bound(k)
+
+
+def opposed(kind: str, m: int, k: int, n: int, g):
+    """Operands whose large elements meet small ones, or none, on the other side, down to subnormal numbers."""
+    a, b = torch.empty(m, k, device="cuda").normal_(generator=g), torch.empty(n, k, device="cuda").normal_(generator=g)
+    sign = 1.0 - 2.0 * (torch.arange(k, device="cuda") % 2)
+    if kind == "decades":        # the odd and the even columns up to 34 decades apart, the other way round in the other operand
+        a *= torch.pow(10.0, torch.linspace(0, 17, m, device="cuda")[:, None] * sign)
+        b *= torch.pow(10.0, -torch.linspace(0, 17, n, device="cuda")[:, None] * sign)
+    elif kind == "shadowed":     # one element each that towers over its row and meets a zero
+        a[:, 40], b[:, 40], a[:, 77], b[:, 77] = 1e12, 0.0, 0.0, 1e12
+    elif kind == "last":         # the same in the last column, after the row's scale has settled, and for some rows only
+        a[::3, k - 1], b[:, k - 1] = 1e15, 0.0
+    elif kind == "subnormal":
+        a *= 1e-37
+        a[:, ::2] *= 1e-3
+        a[::5] *= 1e-3
+        b *= 1e25
+    return a, b
+
+
+@pytest.mark.parametrize("m,k,n", [(9700, 132, 57), (9601, 576, 96), (4800, 160, 129), (1024, 1332, 330), (1029, 2304, 128)])
+@pytest.mark.parametrize("kind", ["decades", "shadowed", "last", "subnormal"])
+def test_opposed_ranges(ops, m, k, n, kind):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(m + k)
+    a, b = opposed(kind, m, k, n, g)
+    got = ops.MultiplyMatrixByTransposedMatrix(a, b)
+    assert worst(got, a, b) < bound(k)
+    bias = torch.empty(n, device="cuda").normal_(generator=g)
+    got = ops.MultiplyMatrixByTransposedMatrix(a, b, free_term=bias)
+    assert worst(got, a, b, extra=bias.expand(m, n)) < bound(k)
+
+
+@pytest.mark.parametrize("shape,k,r,stride,pad,dil", [((5, 45, 47, 64), 70, 3, 1, 1, 1), ((3, 61, 59, 32), 128, 5, 2, 2, 1),
+                                                      ((9, 31, 33, 32), 96, 3, 1, 2, 2), ((4, 75, 90, 3), 64, 7, 2, 3, 1),
+                                                      ((5, 60, 70, 4), 40, 5, 1, 2, 1), ((6, 14, 14, 512), 160, 3, 1, 1, 1)])
+@pytest.mark.parametrize("decades", [6, 15])
+def test_convolutions_of_opposed_ranges(ops, shape, k, r, stride, pad, dil, decades):
+    """The same through im2col, row windows (3 and 4 channels) and split K (the last): channels of opposed magnitude."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(k)
+    x, f = torch.empty(shape, device="cuda").normal_(generator=g), torch.empty(k, r, r, shape[3], device="cuda").normal_(generator=g)
+    scale = torch.pow(10.0, decades * (1.0 - 2.0 * (torch.arange(shape[3], device="cuda") % 2)))
+    x, f = x * scale, f / scale
+    f[1] = 0.0                                    # a filter of zeros
+    got = ops.BlobConvolution(x, f, padding=(pad, pad), stride=(stride, stride), dilation=(dil, dil))
+    conv = lambda p, q: torch.nn.functional.conv2d(p.double().permute(0, 3, 1, 2), q.double().permute(0, 3, 1, 2), stride=stride,
+                                                   padding=pad, dilation=dil).permute(0, 2, 3, 1)
+    size = conv(x.abs(), f.abs())
+    assert bool((got[size == 0] == 0).all())
+    assert float(((got.double() - conv(x, f)).abs() / size.clamp_min(1e-300)).max()) < bound(r * r * shape[3])
 
 
 def test_batches_and_infinities(ops):
