@@ -111,9 +111,10 @@ _lib = None
 class Nb200Error(RuntimeError):
     def __init__(self, fn: str, code: int):
         self.code = code
-        msg = load().nb200_error_string(code).decode() if _lib is not None else str(code)
-        if code in (ELAUNCH, ENODEVICE) and _lib is not None:
-            msg += ": " + _lib.nb200_last_cuda_error().decode()
+        lib = load()  # the failing call may have been the process's first and come through the native half of ops.py
+        msg = lib.nb200_error_string(code).decode()
+        if code in (ELAUNCH, ENODEVICE):
+            msg += ": " + lib.nb200_last_cuda_error().decode()
         super().__init__(f"{fn} failed: {msg} ({code})")
 
 

@@ -18,6 +18,14 @@ def test_native_calls_decline_other_tensors():
         native.transpose(1, a)
 
 
+def test_first_error_of_a_process_has_its_text(monkeypatch):
+    """A native call does not go through capi.load(); an error that it answers is spelled out all the same."""
+    monkeypatch.setattr(ops.capi, "_lib", None)
+    with pytest.raises(ops.capi.Nb200Error, match=r"BlobConvolution failed: .*launch.*: .*\(-3\)") as e:
+        ops._checked("BlobConvolution", ops.capi.ELAUNCH)
+    assert e.value.code == ops.capi.ELAUNCH
+
+
 @pytest.mark.gpu
 def test_errors_are_the_python_codes():
     x, f = torch.zeros(1, 5, 5, 4, device="cuda"), torch.zeros(2, 3, 3, 4, device="cuda")
