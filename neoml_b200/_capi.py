@@ -10,6 +10,15 @@ from pathlib import Path
 
 LIB_PATH = Path(__file__).resolve().parent / "lib" / "libneoml_b200.so"
 
+
+def native_path() -> Path:
+    """The native half of ops.py.  It is compiled against one torch and one interpreter, which its name states: another
+    torch does not load it."""
+    import sysconfig
+    import torch
+    return LIB_PATH.parent / f"_ops_native-torch{torch.__version__}{sysconfig.get_config_var('EXT_SUFFIX')}"
+
+
 OK, EINVAL, ENODEVICE, ELAUNCH, EDEVICE, ETOOBIG = 0, -1, -2, -3, -4, -5
 PREC_3XTF32, PREC_TF32, PREC_FP32_SIMT = 0, 1, 2
 ACT_NONE, ACT_RELU, ACT_HSWISH = 0, 1, 2

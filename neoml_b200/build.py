@@ -1,7 +1,8 @@
 """Builds the native parts of the package in-tree.
 
   neoml_b200/lib/libneoml_b200.so      CUDA kernels + C ABI (include/neoml_b200.h), sm_100a only
-  neoml_b200/lib/_ops_native.so        the native half of neoml_b200/ops.py
+  neoml_b200/lib/_ops_native-*.so      the native half of neoml_b200/ops.py, for this torch and interpreter (only where
+                                       the interpreter's headers are installed; ops.py does without it otherwise)
   neoml_b200/lib/libNeoMathEngineB200.so  C++ IMathEngine implementation over that C ABI; compiled against the
                                        NeoMathEngine headers of a NeoML checkout ($NEOML_REFERENCE_DIR), so it is
                                        only (re)built where such a checkout exists
@@ -121,11 +122,14 @@ def build_engine(verbose: bool = False) -> Path | None:
     return out
 
 
-def build_bindings(verbose: bool = False) -> Path:
+def build_bindings(verbose: bool = False) -> Path | None:
     """g++ build of the native half of neoml_b200/ops.py (a CPython module over torch's headers and the C ABI)."""
     import sysconfig
     import torch
-    src, out = ROOT / "bindings" / "ops_native.cpp", LIB / "_ops_native.so"
+    from neoml_b200._capi import native_path
+    src, out = ROOT / "bindings" / "ops_native.cpp", native_path()
+    if not (Path(sysconfig.get_paths()["include"]) / "Python.h").exists():
+        return out if out.exists() else None
     if not _newer(src, out, sorted(INCLUDE.glob("*.h"))):
         return out
     base = Path(torch.__file__).resolve().parent

@@ -10,6 +10,7 @@ from __future__ import annotations
 import ctypes as C
 import importlib.machinery
 import importlib.util
+import warnings
 
 import torch
 
@@ -20,18 +21,28 @@ from ._capi import (ACT_HSWISH, ACT_NONE, ACT_RELU, PREC_3XTF32, PREC_FP32_SIMT,
 _native_module = None
 
 
+class _DeclinesAll:
+    """In the place of a native half that has not been built for this interpreter and torch."""
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
 def _native():
     """The native half of the calls below (bindings/ops_native.cpp): it answers None for arguments that it does not take,
-    and the Python code after the call then raises or handles them."""
+    and the Python code after the call then raises or handles them.  Its file is named after the torch and the interpreter
+    that it was compiled for; without it the Python code makes every call, with the same kernels and more host time."""
     global _native_module
     if _native_module is None:
-        path = capi.LIB_PATH.parent / "_ops_native.so"
-        if not path.exists():
-            raise RuntimeError(f"{path} is missing: run `python -m neoml_b200.build` (no fallback exists)")
-        loader = importlib.machinery.ExtensionFileLoader("_ops_native", str(path))
-        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_ops_native", loader))
-        loader.exec_module(module)
-        _native_module = module
+        capi.load()
+        path = capi.native_path()
+        if path.exists():
+            loader = importlib.machinery.ExtensionFileLoader("_ops_native", str(path))
+            module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_ops_native", loader))
+            loader.exec_module(module)
+            _native_module = module
+        else:
+            warnings.warn(f"{path} is missing: calls take 10 us longer (python -m neoml_b200.build makes it)")
+            _native_module = _DeclinesAll()
     return _native_module
 
 

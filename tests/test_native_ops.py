@@ -26,6 +26,33 @@ def test_first_error_of_a_process_has_its_text(monkeypatch):
     assert e.value.code == ops.capi.ELAUNCH
 
 
+def test_calls_without_the_native_half(monkeypatch):
+    """Where it has not been built for this torch the Python code behind each call serves (and checks its arguments)."""
+    a = torch.zeros(4, 8)
+    monkeypatch.setattr(torch, "__version__", "0.0")
+    monkeypatch.setattr(ops, "_native_module", None)
+    monkeypatch.setattr(ops, "_stream", lambda: 0)
+    with pytest.warns(UserWarning, match="torch0.0"):
+        assert ops._native().transpose(1, a, 2, 1, 2, 8, None) is None
+    with pytest.raises(AssertionError, match="device-resident"):
+        ops.MultiplyMatrixByTransposedMatrix(a, a)
+
+
+@pytest.mark.gpu
+def test_same_results_without_the_native_half(monkeypatch):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+    a, f = torch.empty(3, 20, 36, device="cuda").normal_(generator=g), torch.empty(5, 3, 3, 36, device="cuda").normal_(generator=g)
+    calls = [lambda: ops.BlobConvolution(a.view(1, 6, 10, 36), f), lambda: ops.MultiplyMatrixByTransposedMatrix(a[0], a[1]),
+             lambda: ops.BatchMultiplyMatrixByTransposedMatrix(a, a), lambda: ops.MultiplyMatrixByMatrix(a[:, :, :20].contiguous(), a),
+             lambda: ops.TransposeMatrix(3, a, 20, 1, 36, 1), lambda: ops.vector_op("EXP", a)]
+    native = [call() for call in calls]
+    monkeypatch.setattr(ops, "_native_module", ops._DeclinesAll())
+    for call, want in zip(calls, native):
+        got = call()
+        assert got.shape == want.shape and torch.equal(got, want)
+
+
 @pytest.mark.gpu
 def test_errors_are_the_python_codes():
     x, f = torch.zeros(1, 5, 5, 4, device="cuda"), torch.zeros(2, 3, 3, 4, device="cuda")
