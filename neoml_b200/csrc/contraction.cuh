@@ -152,7 +152,7 @@ int launch_contraction_tc(const ContractionParams& p, int batch, cudaStream_t st
 TileDivs tile_divs(const ContractionParams& p, long long nTiles, long long tilesPerBatch);
 int launch_contraction_split(const ContractionParams& p, int batch, cudaStream_t stream);
 int contraction_tile_width(int n);
-int balanced_tile_width(long long mTiles, int n, int batch);
+int balanced_tile_width(const ContractionParams& p, long long mTiles, int batch);
 // Tensor maps (CUtensorMap behind the void pointer), contraction_tc.cu
 bool make_rows_map(void* map, const float* base, int k, long long rows, long long ld, int batch, long long batchStride, int boxRows);
 int make_operand_map(void* map, const ContractionParams& p, int batch, int boxRows);

@@ -1014,7 +1014,7 @@ int launch_contraction_split(const ContractionParams& p, int batch, cudaStream_t
 	if(p.M <= 0 || p.N <= 0 || batch <= 0) return NB200_OK;
 	const int tileM = p.a_mode == A_CONV_WINDOW && p.tileM > 0 && p.tileM <= BM ? p.tileM : BM;
 	const bool maySplit = p.splitScratch != nullptr && batch == 1 && p.K >= 8 * BK;
-	switch(maySplit ? contraction_tile_width(p.N) : balanced_tile_width((p.M + tileM - 1LL) / tileM, p.N, batch)) {
+	switch(maySplit ? contraction_tile_width(p.N) : balanced_tile_width(p, (p.M + tileM - 1LL) / tileM, batch)) {
 		case 32: return launch_bn<32>(p, batch, stream);
 		case 64: return launch_bn<64>(p, batch, stream);
 		case 96: return launch_bn<96>(p, batch, stream);

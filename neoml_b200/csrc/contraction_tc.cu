@@ -1301,21 +1301,26 @@ int contraction_tile_width(int n)
 	return best;
 }
 
-// The same where K is not split: the width whose waves over the SMs cost least.  A tile's K block is bound by the copies and
-// the conversion of A far more than by its columns: 128, 96, 64 and 32 of them measured 100 : 90 : 80 : 62 per wave with
-// either kernel (2048 x 1024 x 1300: 56, 51, 63, 86 us in 2, 2, 3, 5 waves).  The least-padded width made such a product
-// 32 columns wide: 1300 columns 86 us for 51, 20000 x 512 x 384 has 4 waves of 128 at 37 us against 13 of 32 at 81,
-// 100000 x 24 x 144 31 us for 25.
-int balanced_tile_width(long long mTiles, int n, int batch)
+// The same where K is not split: the width whose waves over the SMs cost least.  A wave takes a time for its stores, which
+// grows with its columns, and one per K block, which hardly does (the copies and the conversion of A): in units of 10 ns,
+// fitted to 150 products of 3000 to 60000 rows, 64 to 1300 columns and K = 16 to 1024, every width timed.  Result rows that
+// are no whole 16-byte pieces are stored element by element, three to five times as slowly.  Slower than the best width by
+// 1.2 % on average at K <= 32, 0.2 to 1 % beyond, by 13 % at most; the least-padded width by 4 to 10 % at K <= 32, 10 to 15 %
+// at 64 and 128, 16 to 35 % beyond (1300 columns become 32 wide: 2048 x 1024 x 1300 86 us for 51), fixed costs per wave of
+// 100 : 90 : 80 : 62 by 6 to 13 % at K <= 32 (60000 x 24 x 130: 65.5 us, 53 here; 60000 x 32 x 576: 44.5, 38.3 here).
+int balanced_tile_width(const ContractionParams& p, long long mTiles, int batch)
 {
 	const int widths[4] = { 128, 96, 64, 32 };
-	const long long cost[4] = { 100, 90, 80, 62 };
+	const long long stores[2][4] = { { 1225, 900, 580, 255 }, { 250, 172, 125, 86 } };
+	const long long perBlock[2][4] = { { 30, 30, 30, 30 }, { 45, 44, 43, 37 } };
+	const int vec = p.c_vec != 0 && p.accumulate == 0 ? 1 : 0;
+	const long long numKb = (p.K + BK - 1) / BK;
 	const int sms = sm_count();
 	int best = 128;
 	long long least = -1;
 	for(int i = 0; i < 4; ++i) {
-		const long long tiles = mTiles * ((n + widths[i] - 1) / widths[i]) * batch;
-		const long long total = (tiles + sms - 1) / sms * cost[i];
+		const long long tiles = mTiles * ((p.N + widths[i] - 1) / widths[i]) * batch;
+		const long long total = (tiles + sms - 1) / sms * (stores[vec][i] + numKb * perBlock[vec][i]);
 		if(least < 0 || total < least) { least = total; best = widths[i]; }
 	}
 	return best;
@@ -1329,7 +1334,7 @@ int launch_contraction_tc(const ContractionParams& p, int batch, cudaStream_t st
 	// (with room for split K, a few-tile launch keeps the least-padded width: its parts fill the machine whatever the width)
 	const bool maySplit = p.splitScratch != nullptr && batch == 1 && p.K >= 8 * BK;
 	const long long mTiles = (p.M + BM - 1LL) / BM;
-	switch(maySplit ? contraction_tile_width(p.N) : balanced_tile_width(mTiles, p.N, batch)) {
+	switch(maySplit ? contraction_tile_width(p.N) : balanced_tile_width(p, mTiles, batch)) {
 		case 32: return launch_bn<32>(p, batch, stream);
 		case 64: return launch_bn<64>(p, batch, stream);
 		case 96: return launch_bn<96>(p, batch, stream);

@@ -206,3 +206,18 @@ def test_odd_depths(ops, batch, m, k, n, same, precision):
     odd = torch.nn.functional.pad(a[0], (0, 2)).contiguous()     # an odd row length in memory, too
     wide = ops.MultiplyMatrixByTransposedMatrix(odd, b[0], first_width=k, precision=precision, first_row_size=k + 2)
     assert worst(wide, a[0], b[0]) < limit
+
+
+# unsplit products of few K blocks: the tile width follows from the waves, the K blocks and whether result rows are whole 16-byte
+# pieces (here 96, 96, 64, 128 and then 32 columns, most with a remainder)
+@pytest.mark.parametrize("m,k,n", [(20000, 32, 576), (20001, 16, 1300), (60000, 32, 320), (18900, 128, 250 * 4), (20000, 24, 130),
+                                   (3000, 16, 259), (9001, 100, 64), (300, 20, 33)])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_tile_widths(ops, m, k, n, precision):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(m)
+    a, b = torch.empty(m, k, device="cuda").normal_(generator=g), torch.empty(n, k, device="cuda").normal_(generator=g)
+    res = torch.empty(m, n, device="cuda").normal_(generator=g)
+    got = ops.MultiplyMatrixByTransposedMatrix(a, b, residual=res, precision=precision)
+    # 8 products at a time; plain TF32 rounds both operands to 11 bits
+    assert worst(got, a, b, extra=res) < 2 * bound(k) + (2.0 ** -10 if precision else 0.0)
