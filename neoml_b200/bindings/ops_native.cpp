@@ -107,7 +107,7 @@ PyObject* guarded(Py_ssize_t n, Py_ssize_t expected, F&& f)
 	} catch(const NotHere&) {
 		Py_RETURN_NONE;
 	} catch(const c10::OutOfMemoryError&) {
-		Py_RETURN_NONE; // the Python code's allocation raises torch's own error
+		Py_RETURN_NONE; // the Python code does without the work space, or raises torch's own error
 	} catch(const std::exception& e) {
 		PyErr_SetString(PyExc_RuntimeError, e.what());
 		return nullptr;

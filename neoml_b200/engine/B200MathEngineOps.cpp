@@ -534,18 +534,19 @@ int CB200MathEngine::productWithScratch( int batchSize, const float* first, int 
 	const float* prepared = batchSize == 1 && secondAllocation != nullptr
 		? preparedSecondFor( secondAllocation, second, firstHeight, secondHeight, firstWidth, secondRowSize ) : nullptr;
 	const size_t floats = nb200_matrix_product_scratch_floats( batchSize, firstHeight, secondHeight, firstWidth, secondRowSize );
-	if( floats == 0 ) {
+	// (not through this class's StackAlloc, which raises: where there is no room, such as for the copies of operands of odd
+	// depth, the product runs without, more slowly)
+	float* const room = floats > 0 ? static_cast<float*>( memory.StackAlloc( floats * sizeof( float ) ) ) : nullptr;
+	if( room == nullptr && prepared == nullptr ) {
 		return nb200_multiply_matrix_by_transposed_matrix_with_scratch( stream, batchSize, first, firstHeight, firstWidth,
 			firstRowSize, second, secondHeight, secondRowSize, result, resultRowSize, nullptr, epi, precision );
 	}
-	CMemoryHandle scratch = self->StackAlloc( floats * sizeof( float ) );
-	float* const room = static_cast<float*>( CMemoryHandleInternal::GetRaw( scratch ) );
 	const int rc = prepared != nullptr
 		? nb200_multiply_matrix_by_transposed_matrix_prepared( stream, first, firstHeight, firstWidth, firstRowSize, second,
 			secondHeight, secondRowSize, result, resultRowSize, prepared, room, epi, precision )
 		: nb200_multiply_matrix_by_transposed_matrix_with_scratch( stream, batchSize, first, firstHeight, firstWidth,
 			firstRowSize, second, secondHeight, secondRowSize, result, resultRowSize, room, epi, precision );
-	self->StackFree( scratch ); // stream order keeps the kernels ahead of the next user of the stack
+	if( room != nullptr ) self->StackFree( CMemoryHandleInternal::Create( self, room ) ); // stream order keeps the kernels ahead of the next user of the stack
 	return rc;
 }
 

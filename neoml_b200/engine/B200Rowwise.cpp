@@ -455,7 +455,8 @@ void CB200MathEngine::MobileNetV3PreSEBlock( const CBlobDesc& inputDesc, const C
 	}
 	float* expanded = WorkAlloc( static_cast<size_t>( rows ) * d.c );
 	const size_t scratchFloats = nb200_matrix_product_scratch_floats( 1, rows, d.c, inputChannels, inputChannels );
-	float* scratch = scratchFloats > 0 ? WorkAlloc( scratchFloats ) : nullptr;
+	// none where there is no room for it: the product runs without, more slowly
+	float* scratch = scratchFloats > 0 ? static_cast<float*>( memory.Alloc( scratchFloats * sizeof( float ) ) ) : nullptr;
 	nb200_epilogue epi = {};
 	epi.bias = expandFreeTerm != nullptr ? raw( *expandFreeTerm ) : nullptr;
 	epi.act = expandTail.act;
@@ -497,7 +498,7 @@ void CB200MathEngine::MobileNetV3PostSEBlock( const CBlobDesc& channelwiseOutput
 		raw( squeezeAndExciteHandle ), tail.act, tail.param, scaled );
 	if( rc == 0 ) {
 		const size_t scratchFloats = nb200_matrix_product_scratch_floats( 1, rows, outputChannels, channels, channels );
-		float* scratch = scratchFloats > 0 ? WorkAlloc( scratchFloats ) : nullptr;
+		float* scratch = scratchFloats > 0 ? static_cast<float*>( memory.Alloc( scratchFloats * sizeof( float ) ) ) : nullptr;
 		nb200_epilogue epi = {};
 		epi.bias = downFreeTermHandle != nullptr ? raw( *downFreeTermHandle ) : nullptr;
 		if( residualHandle != nullptr ) { epi.residual = raw( *residualHandle ); epi.ld_residual = outputChannels; }

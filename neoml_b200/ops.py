@@ -68,6 +68,16 @@ def _f32(t: torch.Tensor) -> torch.Tensor:
     return t
 
 
+def _product_scratch(need: int, device) -> torch.Tensor | None:
+    """Work space of a matrix product, or None where there is no room for it: the product then runs without, more slowly."""
+    if not need:
+        return None
+    try:
+        return torch.empty(need, dtype=torch.float32, device=device)
+    except torch.cuda.OutOfMemoryError:
+        return None
+
+
 def _epilogue(bias=None, residual=None, ld_residual=0, act=ACT_NONE, act_param=0.0, accumulate=False,
               act_param_device=None):
     return capi.Epilogue(_ptr(bias), _ptr(residual), ld_residual, act, float(act_param), int(accumulate),
@@ -101,9 +111,8 @@ def MultiplyMatrixByTransposedMatrix(first, second, result=None, *, first_row_si
         result = torch.empty((m, ldc), dtype=torch.float32, device=first.device)
     epi = _epilogue(free_term, residual, ldc, act, act_param, accumulate)
     lib = capi.load()
-    need = lib.nb200_matrix_product_scratch_floats(1, m, n, k, ldb) if use_scratch else 0
-    if need:
-        scratch = torch.empty(need, dtype=torch.float32, device=first.device)
+    scratch = _product_scratch(lib.nb200_matrix_product_scratch_floats(1, m, n, k, ldb) if use_scratch else 0, first.device)
+    if scratch is not None:
         capi.check("MultiplyMatrixByTransposedMatrix", lib.nb200_multiply_matrix_by_transposed_matrix_with_scratch(
             _stream(), 1, _ptr(_f32(first)), m, k, lda, _ptr(_f32(second)), n, ldb, _ptr(result), ldc, _ptr(scratch),
             C.byref(epi), precision))
@@ -128,9 +137,8 @@ def BatchMultiplyMatrixByTransposedMatrix(first, second, result=None, *, precisi
 
 def _batch_mmt(b, first, m, k, second, n, result, precision, use_scratch):
     lib = capi.load()
-    need = lib.nb200_matrix_product_scratch_floats(b, m, n, k, k) if use_scratch else 0
-    if need:
-        scratch = torch.empty(need, dtype=torch.float32, device=first.device)
+    scratch = _product_scratch(lib.nb200_matrix_product_scratch_floats(b, m, n, k, k) if use_scratch else 0, first.device)
+    if scratch is not None:
         capi.check("BatchMultiplyMatrixByTransposedMatrix", lib.nb200_multiply_matrix_by_transposed_matrix_with_scratch(
             _stream(), b, _ptr(first), m, k, k, _ptr(second), n, k, _ptr(result), n, _ptr(scratch), None, precision))
     else:

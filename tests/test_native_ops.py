@@ -54,6 +54,31 @@ def test_same_results_without_the_native_half(monkeypatch):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("native", [True, False])
+def test_products_where_work_space_does_not_fit(monkeypatch, native):
+    """Odd depths want copies of both operands; without room for them the product is gathered, as it is without work space."""
+    if not native:
+        monkeypatch.setattr(ops, "_native_module", ops._DeclinesAll())
+    g = torch.Generator(device="cuda")
+    g.manual_seed(2)
+    a, b = torch.empty(1, 20000, 1001, device="cuda").normal_(generator=g), torch.empty(1, 300, 1001, device="cuda").normal_(generator=g)
+    want, batched = torch.empty(20000, 300, device="cuda"), torch.empty(1, 20000, 300, device="cuda")
+    got = torch.empty_like(want)
+    ops.MultiplyMatrixByTransposedMatrix(a[0], b[0], want, use_scratch=False)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    try:
+        # half of what the copies take
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (40 << 20)) / total)
+        ops.MultiplyMatrixByTransposedMatrix(a[0], b[0], got)
+        ops.BatchMultiplyMatrixByTransposedMatrix(a, b, batched)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert torch.equal(got, want) and torch.equal(batched[0], want)
+
+
+@pytest.mark.gpu
 def test_errors_are_the_python_codes():
     x, f = torch.zeros(1, 5, 5, 4, device="cuda"), torch.zeros(2, 3, 3, 4, device="cuda")
     y = ops.BlobConvolution(x, f)
