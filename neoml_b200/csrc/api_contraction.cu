@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(256) prepare_filter_kernel(const float* __rest
 }
 
 // The operands of a product whose rows are not whole 16-byte pieces (an odd depth), copied into rows that are: y[r][0..k) of
-// rows k4 floats apart = x[r][0..k) of rows ld apart; the floats between k and k4 are never read.  A warp per row, both
+// rows k4 floats apart = x[r][0..k) of rows ld apart, zeros between k and k4.  A warp per row, both
 // operands in one launch.  Bound: memory (4-byte accesses, each row coalesced).  It buys the TMA-fed kernels: their
 // cp.async twin fetches such rows float by float, 5.9 us per K block of 128 x 96 tiles whatever their number below a wave.
 // Both operands copied and multiplied against gathered: 5 x (333 x 517 x 259) 25.7 us against 99.9, 2000 x 1003 x 1005 47.6
@@ -126,6 +126,7 @@ __global__ void __launch_bounds__(256) repack_rows_kernel(const RepackRows first
 		float* dst = (inFirst ? first.y : second.y) + row * k4;
 #pragma unroll 8
 		for(int i = lane; i < k; i += 32) dst[i] = __ldg(src + i);
+		if(lane < k4 - k) dst[k + lane] = 0.f; // outside every tile, but prepare_filter_kernel passes over whole rows
 	}
 }
 
