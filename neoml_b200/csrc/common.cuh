@@ -116,18 +116,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity)
 	return done != 0;
 }
 
-// One look at the barrier, without waiting; the lanes of a converged warp agree on the answer.
-__device__ __forceinline__ bool mbar_test_warp(uint64_t* bar, uint32_t parity)
-{
-	uint32_t done;
-	asm volatile(
-		"{\n\t.reg .pred P;\n\t"
-		"mbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
-		"selp.b32 %0, 1, 0, P;\n\t}"
-		: "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-	return __all_sync(0xffffffffu, done != 0) != 0;
-}
-
 __device__ __forceinline__ uint64_t global_timer_ns()
 {
 	uint64_t t;
@@ -276,6 +264,7 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r)
 		  "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
 		: "memory");
 }
+// 8 consecutive columns, issue only (tmem_ld_wait() before the first use)
 __device__ __forceinline__ void tmem_ld8_issue(uint32_t taddr, uint32_t* r)
 {
 	asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"

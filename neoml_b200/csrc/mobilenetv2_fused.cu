@@ -89,14 +89,6 @@ __device__ __forceinline__ Act<HSWISH> make_act(int kind, float param)
 	return a;
 }
 
-// 32 lanes x 32 bit, 8 consecutive columns, issue only (tmem_ld_wait() before the first use)
-__device__ __forceinline__ void tmem_ld8_issue_local(uint32_t taddr, uint32_t* r)
-{
-	asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-		: "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-		: "r"(taddr));
-}
-
 template<bool VALUE>
 struct Flag {
 	static constexpr bool value = VALUE;
@@ -399,9 +391,9 @@ __global__ void __launch_bounds__(THREADS, 1) mbv2_fused_kernel(const FusedParam
 				uint32_t raw[56], last[24];
 				tmem_ld32_issue(src, raw);
 				tmem_ld16_issue(src + 32, raw + 32);
-				tmem_ld8_issue_local(src + 48, raw + 48);      // halo rows 0..2 are columns 0..53
+				tmem_ld8_issue(src + 48, raw + 48);            // halo rows 0..2 are columns 0..53
 				tmem_ld16_issue(src + 54, last);                // halo row 3: columns 54..69 ...
-				tmem_ld8_issue_local(src + 64, last + 16);      // ... and 70, 71 (elements 6, 7 of this piece)
+				tmem_ld8_issue(src + 64, last + 16);            // ... and 70, 71 (elements 6, 7 of this piece)
 				// which halo pixels lie inside the image: bit hx of rowBits[hy] (the same for every lane)
 				uint32_t colBits = 0;
 #pragma unroll
