@@ -221,3 +221,33 @@ def test_tile_widths(ops, m, k, n, precision):
     got = ops.MultiplyMatrixByTransposedMatrix(a, b, residual=res, precision=precision)
     # 8 products at a time; plain TF32 rounds both operands to 11 bits
     assert worst(got, a, b, extra=res) < 2 * bound(k) + (2.0 ** -10 if precision else 0.0)
+
+
+@pytest.mark.parametrize("shape,k,r,stride,pad", [((5, 45, 47, 64), 70, 3, 1, 1), ((9, 40, 40, 160), 96, 1, 1, 0),
+                                                  ((4, 75, 90, 3), 64, 7, 2, 3), ((6, 14, 14, 512), 160, 3, 1, 1)])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_prepared_filters(ops, shape, k, r, stride, pad, precision):
+    """A filter prepared once (im2col, plain rows, row windows, split K) gives the bits of one prepared in the call, and its other
+    form serves a single image, which the TF32 kernel takes."""
+    capi, lib = ops.capi, ops.capi.load()
+    g = torch.Generator(device="cuda")
+    g.manual_seed(k)
+    x, f = torch.empty(shape, device="cuda").normal_(generator=g), torch.empty(k, r, r, shape[3], device="cuda").normal_(generator=g)
+    bias = torch.empty(k, device="cuda").normal_(generator=g)
+    ho, wo = (ops.conv_output_size(v, r, pad, stride) for v in shape[1:3])
+    desc = lambda n: capi.ConvDesc(n, *shape[1:], k, r, r, pad, pad, stride, stride, 1, 1, ho, wo)
+    stream, epi = torch.cuda.current_stream().cuda_stream, capi.Epilogue(bias.data_ptr(), None, k, capi.ACT_NONE, 0.0, 0, None)
+    prepared = torch.empty(lib.nb200_blob_convolution_prepared_filter_floats(desc(shape[0])), device="cuda")
+    capi.check("prepare", lib.nb200_blob_convolution_prepare_filter(stream, desc(shape[0]), f.data_ptr(), prepared.data_ptr(), precision))
+    for n in (shape[0], 1):
+        y = torch.empty(n, ho, wo, k, device="cuda")
+        scratch = torch.empty(lib.nb200_blob_convolution_scratch_floats(desc(n)) + 1, device="cuda")
+        capi.check("convolution", lib.nb200_blob_convolution_with_prepared_filter(
+            stream, desc(n), x.data_ptr(), f.data_ptr(), prepared.data_ptr(), y.data_ptr(), scratch.data_ptr(), epi, precision))
+        if n == shape[0]:
+            assert torch.equal(y, ops.BlobConvolution(x, f, bias, padding=(pad, pad), stride=(stride, stride), precision=precision))
+        conv = lambda p, q: torch.nn.functional.conv2d(p.double().permute(0, 3, 1, 2), q.double().permute(0, 3, 1, 2), stride=stride,
+                                                       padding=pad).permute(0, 2, 3, 1)
+        err = (y.double() - conv(x[:n], f) - bias.double()).abs() / (conv(x[:n].abs(), f.abs()) + bias.abs().double())
+        # the TF32 kernel accumulates 8 products at a time; plain TF32 rounds both operands to 11 bits
+        assert float(err.max()) < 2 * bound(r * r * shape[3]) + (2.0 ** -10 if precision else 0.0)
