@@ -158,8 +158,8 @@ size_t prepared_filter_floats(long long k, long long r, long long s, long long c
 // a few K blocks per part and a finishing pass in either kernel: 4116 rows x 256 columns took 12.9 / 13.0 us at K = 256, 16.0 /
 // 15.0 at 576, 18.1 / 16.2 at 768, 32.8 / 25.5 at 2304, 1029 x 512 13.3 / 14.5 at 384 and 14.8 / 14.0 at 768.  It goes there
 // from 24 K blocks on, where the gain is clear of the spread at every size tried; below, a launch keeps the bits of the
-// kernel that gathers its operands.  Deeper products than 2^18 stay on the TF32 kernel: a tile of them whose sums all had to be
-// formed anew (contraction_split.cu, small_sums) would come near the two seconds after which a wait gives up.
+// kernel that gathers its operands.  Deeper products than 2^18 stay on the TF32 kernel: a tile whose sums
+// all have to be formed anew (contraction_split.cu, sums_anew) takes 64 ms at K = 2^16, and a wait gives up after two seconds.
 bool split_form_pays(long long mTiles, long long n, long long k, long long batch)
 {
 	const int width = contraction_tile_width(static_cast<int>(n));

@@ -23,10 +23,12 @@
 // S = sum |a||b| in scaled units, K * 2^-20 <= K * 2^-25 * S wherever S >= 2^5, as much as the accumulation of three TF32
 // products may take.  S >= 2^5 follows from a sum of 2^5 or more, and from a main part of 2^5 + K * 2^-8 or more (an element's hi half
 // is larger than the element by 2^-11 of it or by 2^-25 at most).  The sums of which neither holds -- of ordinary operands
-// one in 10^8 -- the epilogue looks into (small_sums): where the row of A or the row of B holds such elements the sum is
+// one in 10^8 -- the epilogue looks into (coarse_rows, sums_anew): where the row of A or the row of B holds such elements the sum is
 // formed anew from the fp32 operands.  That serves rows whose large elements meet small or no ones on the other side
-// (1e6 and 1e-6 by weights of 1e-6 and 1e6: 5e-3 of sum |a||b| without it); a launch of nothing but such sums takes some 15
-// times as long.  The look at every sum costs 1 to 4 % of an ordinary launch; marks of A's rows from the converters, which
+// (1e6 and 1e-6 by weights of 1e-6 and 1e6: 5e-3 of sum |a||b| without it).  A launch
+// of nothing but such sums takes far longer (20000 x 1152 x 128: 2.3 ms for 53 us, 4096 x 4096 x 1024 7.8 ms for 0.12), one of
+// operands so sparse that most sums are zero, whose rows are only looked through, up to twice as long as three TF32
+// products (zeros in 99 % of both: 171 us for 89; 80 % and 95 %: 87 for 90).  The look at every sum costs 1 to 4 % of an ordinary launch; marks of A's rows from the converters, which
 // every block would pay for, cost 10 to 18 %.
 // A row of subnormal numbers alone counts where its first K block holds one.
 //
@@ -191,67 +193,126 @@ __device__ __forceinline__ const float* row_block(const ContractionParams& p, co
 	return A + at.base + (iy * p.W + ix) * p.Cin + c;
 }
 
-// The sums that came out small.  A warp's lane r has the bits of those among the 16 columns from n0 on that belong to row m0 + r;
-// their finished values lie in its 64 bytes of the staging slice.  A row of A is looked through for elements of fewer than
-// 22 bits while its first four columns are formed (`clean`: the rows that have none), rows of B carry the mark in their
-// scale (`markedCols`); a sum with such elements on either side is formed anew: fused multiply-adds of the fp32 operands, 32
-// partial sums along K, subnormal numbers included.  Four columns at a time, as whole tiles of such sums occur in data that
-// is made for it.
-__device__ __forceinline__ void small_sums(const ContractionParams& p, uint32_t small, uint32_t markedCols, float inv, int batch, int m0,
-	int n0, int kbBegin, int kbEnd, uint8_t* stg, uint32_t& clean)
+// How many of a K block's 32 floats belong to the sum: the last block's remainder; windows: the filter's taps.
+__device__ __forceinline__ int floats_in_block(const ContractionParams& p, int kb)
 {
+	return p.a_mode == A_CONV_WINDOW ? p.filterS * p.Cin : min(BK, p.K - kb * BK);
+}
+// Floats 4c .. 4c + 3 of a block at src (16-byte aligned; null: zeros) of which `count` belong to the sum: those that are whole
+// quads.  No branch, so that several are in flight; the others by last_floats().
+__device__ __forceinline__ float4 whole_quad(const float* src, int c, int count)
+{
+	return src != nullptr && 4 * c + 4 <= count ? __ldg(reinterpret_cast<const float4*>(src) + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+}
+__device__ __forceinline__ float4 last_floats(const float* src, int count)
+{
+	float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+	src += count & ~3;
+	if((count & 3) > 0) v.x = __ldg(src);
+	if((count & 3) > 1) v.y = __ldg(src + 1);
+	if((count & 3) > 2) v.z = __ldg(src + 2);
+	return v;
+}
+
+// Which of a warp's rows (bits of `rows`, from row m0 on) hold elements of fewer than 22 bits; lane r has row r's inverse scale.
+// A warp takes four K blocks of a row at a time, four loads ahead: sums that are zero are what sparse operands are full of,
+// and their rows are looked through to no avail.
+__device__ __forceinline__ uint32_t coarse_rows(const ContractionParams& p, uint32_t rows, float inv, int batch, int m0, int kbBegin,
+	int kbEnd)
+{
+	const int lane = threadIdx.x & 31, c = lane & 7;
+	const float* A = p.A + batch * p.strideA;
+	uint32_t coarse = 0;
+#pragma unroll 1
+	for(; rows != 0; rows &= rows - 1) {
+		const int r = __ffs(rows) - 1;
+		const uint32_t below = coarse_below(__shfl_sync(0xffffffffu, inv, r));
+		const ConvRow at = p.a_mode == A_ROWS ? ConvRow{} : conv_row(p, m0 + r);
+		uint32_t smallest = 0xffffffffu;
+#pragma unroll 1
+		for(int first = kbBegin + (lane >> 3); first < kbEnd; first += 16) {
+			float4 v[4];
+#pragma unroll
+			for(int i = 0; i < 4; ++i) {
+				const int kb = min(first + 4 * i, kbEnd - 1);
+				v[i] = whole_quad(row_block(p, A, at, m0 + r, kb), c, floats_in_block(p, kb));
+			}
+#pragma unroll
+			for(int i = 0; i < 4; ++i) smallest = smallest_key(smallest, v[i]);
+		}
+		if(p.a_mode == A_ROWS && (p.K & 3) != 0 && kbEnd * BK >= p.K) {
+			smallest = smallest_key(smallest, last_floats(A + static_cast<size_t>(m0 + r) * p.lda, p.K));
+		}
+		if(__any_sync(0xffffffffu, smallest < below)) coarse |= 1u << r;
+	}
+	return coarse;
+}
+
+__device__ __forceinline__ void fma_full(float& sum, float a, float b) // subnormal numbers included
+{
+	asm("fma.rn.f32 %0, %1, %2, %0;" : "+f"(sum) : "f"(a), "f"(b));
+}
+__device__ __forceinline__ float add_full(float a, float b)
+{
+	asm("add.rn.f32 %0, %0, %1;" : "+f"(a) : "f"(b));
+	return a;
+}
+
+// Forms sums anew from the fp32 operands: those of row m (one per lane) and of the columns n0 + t with bit t in `wanted`.  They
+// replace mine[t].  A lane holds its row's floats of a K block; the columns of B that any lane wants are fetched four at
+// a time, a float per lane, and handed round by shuffles: whole tiles of such sums occur in data that is made for it.
+__device__ __forceinline__ void sums_anew(const ContractionParams& p, uint32_t wanted, int batch, int m, int n0, int kbBegin, int kbEnd,
+	float* mine)
+{
+	const uint32_t columns = __reduce_or_sync(0xffffffffu, wanted);
+	if(columns == 0) return;
 	const int lane = threadIdx.x & 31;
 	const float* A = p.A + batch * p.strideA;
 	const float* B = p.B + batch * p.strideB;
+	const ConvRow at = p.a_mode == A_ROWS || wanted == 0 ? ConvRow{} : conv_row(p, m);
+	// where this lane's float of a K block lies in a row of B, and how far it is to the next block's and the next row's
+	int inBlock = lane, block = BK;
+	long long row = p.ldb;
+	bool there = true;
+	if(p.a_mode == A_CONV_WINDOW) {
+		// the filter as the caller has it: channels and taps that are not there count nothing
+		const int tap = lane / p.Cin, ch = lane - tap * p.Cin;
+		there = tap < p.filterS && ch < p.filterC;
+		inBlock = tap * p.filterC + ch;
+		block = p.filterS * p.filterC;
+		row = static_cast<long long>(p.K / BK) * block;
+	}
 #pragma unroll 1
-	for(uint32_t rows = __ballot_sync(0xffffffffu, small != 0); rows != 0; rows &= rows - 1) {
-		const int r = __ffs(rows) - 1, m = m0 + r;
-		uint32_t cols = __shfl_sync(0xffffffffu, small, r);
-		if(clean >> r & 1u) cols &= markedCols;
-		const uint32_t below = coarse_below(__shfl_sync(0xffffffffu, inv, r));
-		const ConvRow at = p.a_mode == A_ROWS ? ConvRow{} : conv_row(p, m);
+	for(uint32_t w = wanted; w != 0; w &= w - 1) mine[__ffs(w) - 1] = 0.f;
 #pragma unroll 1
-		while(cols != 0) {
-			const int q = (__ffs(cols) - 1) >> 2;
-			float sum[4] = { 0.f, 0.f, 0.f, 0.f };
-			uint32_t smallest = 0xffffffffu;
-#pragma unroll 1
-			for(int kb = kbBegin; kb < kbEnd; ++kb) {
-				const float* src = row_block(p, A, at, m, kb);
-				bool real = src != nullptr && kb * BK + lane < p.K;
-				int b = kb * BK + lane;
-				long long step = p.ldb;
-				if(p.a_mode == A_CONV_WINDOW) {
-					// the filter as the caller has it: channels and taps that are not there count nothing
-					const int tap = lane / p.Cin, ch = lane - tap * p.Cin;
-					real = tap < p.filterS && ch < p.filterC;
-					b = (kb * p.filterS + tap) * p.filterC + ch;
-					step = static_cast<long long>(p.K / BK) * p.filterS * p.filterC;
-				}
-				if(real) {
-					const float a = __ldg(src + lane);
-					smallest = min(smallest, small_key(a));
+	for(int kb = kbBegin; kb < kbEnd; ++kb) {
+		const float* src = wanted != 0 ? row_block(p, A, at, m, kb) : nullptr;
+		const int count = floats_in_block(p, kb);
+		float x[BK];
 #pragma unroll
-					for(int t = 0; t < 4; ++t) {
-						const float w = __ldg(B + min(n0 + 4 * q + t, p.N - 1) * step + b);
-						asm("fma.rn.f32 %0, %1, %2, %0;" : "+f"(sum[t]) : "f"(a), "f"(w));
-					}
-				}
-			}
-			if(!__any_sync(0xffffffffu, smallest < below)) {
-				clean |= 1u << r;
-				cols &= markedCols;
-			}
-			float mine = 0.f; // of column 4 q + lane
+		for(int c = 0; c < 8; ++c) {
+			float4 v = whole_quad(src, c, count);
+			if((count & 3) != 0 && c == count >> 2 && src != nullptr) v = last_floats(src, count);
+			x[4 * c] = v.x; x[4 * c + 1] = v.y; x[4 * c + 2] = v.z; x[4 * c + 3] = v.w;
+		}
+		const bool real = there && kb * BK + lane < p.K;
+		const float* b = B + n0 * row + static_cast<long long>(kb) * block + inBlock;
+#pragma unroll 1
+		for(int q = 0; q < 16; q += 4) {
+			const uint32_t four = (columns >> q) & 15u;
+			if(four == 0) continue;
+			float w[4];
 #pragma unroll
+			for(int t = 0; t < 4; ++t) w[t] = real && ((four >> t) & 1u) ? __ldg(b + (q + t) * row) : 0.f;
+			// (not unrolled: with four copies of the loop below the 128- and 96-column kernels spilled)
+#pragma unroll 1
 			for(int t = 0; t < 4; ++t) {
+				float sum[4] = { 0.f, 0.f, 0.f, 0.f };
 #pragma unroll
-				for(int o = 16; o > 0; o >>= 1) sum[t] += __shfl_xor_sync(0xffffffffu, sum[t], o);
-				if(lane == t) mine = sum[t];
+				for(int i = 0; i < BK; ++i) fma_full(sum[i & 3], x[i], __shfl_sync(0xffffffffu, w[0], i));
+				w[0] = w[1]; w[1] = w[2]; w[2] = w[3];
+				if((wanted >> (q + t)) & 1u) mine[q + t] = add_full(mine[q + t], add_full(add_full(sum[0], sum[1]), add_full(sum[2], sum[3])));
 			}
-			const uint32_t four = (cols >> (4 * q)) & 15u;
-			if((four >> lane) & 1u) reinterpret_cast<float*>(stg + r * 64)[4 * q + lane] = mine;
-			cols &= ~(15u << (4 * q));
 		}
 	}
 }
@@ -665,11 +726,16 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 			// into, ahead of the loop below: rare, and a branch per warp and tile.
 			const bool careful = __any_sync(0xffffffffu, (alive && least < small) || (inv < ROW_INV_MIN && inv != 0.f) || inv > ROW_INV_MAX) != 0;
 			if(__builtin_expect(careful, 0)) {
-				uint32_t clean = 0;
 				float* mine = reinterpret_cast<float*>(stg + lane * 64);
+				const int kbBegin = (work - tileIdx * kSplits) * numKb;
+				// (rows this tiny may have lost subnormal elements in blocks before the scale was set)
+				const bool tiny = inv < 0x1p-90f;
+				const uint32_t suspects = __ballot_sync(0xffffffffu, alive && (least < small || tiny));
+				const uint32_t coarse = coarse_rows(p, suspects, inv, tc.batch, rowBase, kbBegin, kbBegin + numKb);
+				const bool coarseRow = (coarse >> lane & 1u) != 0;
 #pragma unroll 1
 				for(int g = 0; g < HALF_COLS; g += 16) {
-					uint32_t a[16], smallCols = 0, markedCols = 0;
+					uint32_t a[16], wanted = 0;
 					tmem_ld16_issue(accMain + g, a);
 					tmem_ld_wait();
 #pragma unroll
@@ -677,14 +743,10 @@ __global__ void __maxnreg__(REGS_LAUNCH) contraction_split_kernel(const Contract
 #pragma unroll 1
 					for(int i = 0; i < 16; ++i) {
 						const float v = mine[i], scale = scaleStrip[g + i]; // 0: a row of B that is all zeros, or none
-						// (rows this tiny may have lost subnormal elements in blocks before the scale was set)
-						if(alive && scale != 0.f && (fabsf(v) < small || inv < 0x1p-90f)) smallCols |= 1u << i;
-						if(scale < 0.f) markedCols |= 1u << i;
+						if(alive && scale != 0.f && (coarseRow || scale < 0.f) && (fabsf(v) < small || tiny)) wanted |= 1u << i;
 						mine[i] = unscale(v, inv, fabsf(scale));
 					}
-					__syncwarp();
-					const int kbBegin = (work - tileIdx * kSplits) * numKb;
-					small_sums(p, smallCols, markedCols, inv, tc.batch, rowBase, colBase + g, kbBegin, kbBegin + numKb, stg, clean);
+					sums_anew(p, wanted, tc.batch, rowBase + lane, colBase + g, kbBegin, kbBegin + numKb, mine);
 					__syncwarp();
 #pragma unroll
 					for(int q = 0; q < 4; ++q) {
