@@ -49,7 +49,7 @@ def parse_args():
     ap.add_argument("--warmup", type=int, default=3)
     ap.add_argument("--impl", default="ours", choices=["ours", "reference"])
     ap.add_argument("--batch", type=int, default=256, help="per-GPU batch")
-    ap.add_argument("--precision", type=int, default=0, help="0 = 3xTF32 (default), 1 = TF32 opt-in")
+    ap.add_argument("--precision", type=int, default=0, help="0 = fp32 accuracy (default: three products of fp16 or TF32 halves), 1 = TF32 opt-in")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-peak", action="store_true", help="skip the TF32 peak measurement (profiler captures)")
     ap.add_argument("--layers", action="store_true", help="print the per-contraction timing table to stderr")
@@ -378,13 +378,17 @@ def run_ours(args):
     achieved_tf = flops / (tc_ms * 1e-3) / 1e12
     mma_per_product = 3 if args.precision == 0 else 1
     tf32 = None if args.no_peak else measure_tf32_peak(torch)
-    if tf32 is not None:
+    if args.precision == 0:
+        # the large layers run on fp16 halves, whose rate is that of bf16; those of K <= 128 on TF32 halves at half of it
+        eff_peak, eff_src = peak_tf / mma_per_product, "bf16 sustained"
+    elif tf32 is not None:
         eff_peak, eff_src = tf32["sustained_tflops"] / mma_per_product, "TF32 sustained, measured in this run"
     else:
         eff_peak, eff_src = peak_tf / 2 / mma_per_product, "bf16 sustained / 2 (not measured in this run)"
     act_bytes = resnet50.contraction_bytes_per_image() * batch + resnet50.weight_bytes()
     roofline = {
-        "bound": "tensor", "kernel": "contraction_tc_kernel (tcgen05 kind::tf32, implicit-GEMM conv + FC)",
+        "bound": "tensor", "kernel": "contraction_split_kernel (tcgen05 kind::f16) and contraction_tc_kernel (kind::tf32), implicit-GEMM conv + FC"
+        if args.precision == 0 else "contraction_tc_kernel (tcgen05 kind::tf32, implicit-GEMM conv + FC)",
         "achieved": round(achieved_tf, 2), "peak": peak_tf, "unit": "TFLOP/s", "frac": round(achieved_tf / peak_tf, 4),
         "peak_source": peak_src,
         "traffic": round(TRAFFIC_MB_PER_IMAGE * 1e6 * batch / max(tc_launches, 1) / 1e9, 4),
@@ -398,7 +402,7 @@ def run_ours(args):
         "effective_peak_source": f"{eff_src}, / {mma_per_product} MMAs per product",
         "frac_of_effective_peak": round(achieved_tf / eff_peak, 4),
         "whole_step_frac_of_effective_peak": round(flops / (ms_total / args.steps * 1e-3) / 1e12 / eff_peak, 4),
-        "note": "peak is dense bf16; this arithmetic is TF32 (3 MMAs per product in the default 3xTF32 mode), "
+        "note": "peak is dense bf16; by default 3 MMAs per product, of fp16 halves (large layers) or TF32 halves; "
                 "algorithmic flops counted once",
     }
 
@@ -408,7 +412,7 @@ def run_ours(args):
         "metric": METRIC, "value": round(images / (ms_total * 1e-3), 2), "unit": UNIT, "n_gpus": world,
         "steps": args.steps, "warmup": max(args.warmup, 3), "ms_per_step": round(ms_step, 3),
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-        "dtype": "fp32 (3xTF32 split on tcgen05, fp32 accumulate)" if args.precision == 0 else "tf32",
+        "dtype": "fp32 (three products of fp16 or TF32 halves on tcgen05, fp32 accumulate)" if args.precision == 0 else "tf32",
         "data": "synthetic",
         "config": {"workload": WORKLOAD if batch == 256 else f"resnet50_v1.5_infer_b{batch}",
                    "per_gpu_batch": batch, "global_batch": batch * world, "parallelism": f"batch-sharded x{world}",
@@ -520,7 +524,8 @@ def run_transformer(args):
     peaks_path = ROOT / "MEASURED_PEAKS.json"
     peak_tf = float(json.loads(peaks_path.read_text())["bf16_tflops_sustained"]) if peaks_path.exists() else 1390.7
     mma = 3 if args.precision == 0 else 1
-    eff = (tf32["sustained_tflops"] if tf32 else peak_tf / 2) / mma
+    # the products run on fp16 halves by default (the rate of bf16), the attention kernel on TF32 halves
+    eff = peak_tf / mma if args.precision == 0 else (tf32["sustained_tflops"] if tf32 else peak_tf / 2) / mma
     tf = flops / ms / 1e9
     print(json.dumps({"mode": "transformer", "workload": "transformer_encoder_12x_b64_s512_h768 (CDnn::RunOnce)",
                       "ms_per_step": round(ms, 3), "sequences_per_s": round(b / ms * 1e3, 1), "launches_per_step": int(launches),
@@ -626,14 +631,14 @@ def run_ops(args):
 def run_products(args):
     """The dense contractions of configs 1, 2, 4 and 5 at full size: algorithmic flops (2*M*N*K, counted once) over the
     CUDA-event time of the public call (operand preparation and scratch allocation included), against the tensor peak
-    of this arithmetic (measured sustained bf16 / 2 for TF32 / 3 MMAs per product for 3xTF32)."""
+    of this arithmetic (measured sustained bf16 / 3 MMAs per product of fp16 halves; / 2 for the TF32 opt-in)."""
     import torch
     from neoml_b200 import ops
     if not torch.cuda.is_available():
         raise SystemExit("bench.py --products needs a CUDA device: the product path has no CPU fallback")
     peaks_path = ROOT / "MEASURED_PEAKS.json"
     peak = float(json.loads(peaks_path.read_text())["bf16_tflops_sustained"]) if peaks_path.exists() else 1390.7
-    eff = peak / 2 / (3 if args.precision == 0 else 1)
+    eff = peak / (3 if args.precision == 0 else 2)
     dev, prec = "cuda", args.precision
     rnd = lambda *shape: torch.rand(*shape, device=dev) - 0.5
     cases = []   # (name, algorithmic flops, setup): setup() allocates the operands and returns the call to time

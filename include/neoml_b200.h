@@ -37,7 +37,9 @@ enum {
 /* Arithmetic of the dense contractions.  The reference selects cuBLAS math modes with the engine flags
  * GpuMathEngineCublasUseTensorCores{Half,TF32}Flag (NME.h:1271-1274, CudaMathEngine.cu:56-65). */
 enum {
-	NB200_PREC_3XTF32 = 0, /* default: hi/lo TF32 split, 3 tcgen05 MMAs, fp32 accumulate; fp32-level accuracy */
+	NB200_PREC_3XTF32 = 0, /* default, fp32-level accuracy: hi/lo split of both operands, 3 tcgen05 MMAs, fp32 accumulate.  The
+	                        * parts are TF32; in large products whose second operand is prepared they are fp16 with a
+	                        * scale per row, and sums that this could cost bits are formed anew in fp32 */
 	NB200_PREC_TF32 = 1,   /* opt-in single TF32 MMA (1e-2 tolerance class) */
 	NB200_PREC_FP32_SIMT = 2 /* exact fp32 FMA on CUDA cores; diagnostic cross-check, slow */
 };
@@ -90,7 +92,9 @@ NB200_API int nb200_batch_multiply_matrix_by_transposed_matrix(void* stream, int
  * calls: `batch` problems whose operands follow one another (A_b = a + b*m*lda, B_b = b + b*n*ldb, C_b = c + b*m*ldc).
  * `scratch` (NULL = none) holds nb200_matrix_product_scratch_floats(batch, m, n, k, ldb) floats of device memory:
  * for tall products the second operand is split for the tensor core once per call instead of tile by tile in every
- * CTA, and products with few output tiles (a classifier at batch 1) cut their K loop into parts summed in fixed order. */
+ * CTA, and products with few output tiles (a classifier at batch 1) cut their K loop into parts summed in fixed order.
+ * Where rows are no whole 16-byte pieces (k or ldb no multiple of four) the floats include copies of both operands in
+ * rows that are; without scratch such a product is gathered element by element, slower but with no memory of its own. */
 NB200_API size_t nb200_matrix_product_scratch_floats(int batch, int m, int n, int k, int ldb);
 NB200_API int nb200_multiply_matrix_by_transposed_matrix_with_scratch(void* stream, int batch, const float* a, int m,
 	int k, int lda, const float* b, int n, int ldb, float* c, int ldc, float* scratch, const nb200_epilogue* epi,
@@ -99,7 +103,9 @@ NB200_API int nb200_multiply_matrix_by_transposed_matrix_with_scratch(void* stre
  * layer's weights do not change between passes, so their tensor-core forms (for 3xTF32 the lo part of the TF32 split and
  * the scaled fp16 split that tall products run on, for TF32 the rounded copy) are made once -- nb200_matrix_product_prepared_floats(m, n, k, ldb) floats of device memory,
  * 16-byte aligned, 0 when a product of m rows does not use a prepared operand -- and handed to every call until the
- * weights change.  `scratch` then only serves split K (NULL allowed); prepared_b == NULL is the call above. */
+ * weights change.  `scratch`: NULL, or as many floats as for the call above.  It serves split K; where the rows of an
+ * operand are no whole 16-byte pieces it takes copies of both, and the prepared form is not used (nor is it without
+ * scratch: such rows are gathered).  prepared_b == NULL is the call above. */
 NB200_API size_t nb200_matrix_product_prepared_floats(int m, int n, int k, int ldb);
 NB200_API int nb200_matrix_product_prepare_second(void* stream, const float* b, int n, int k, int ldb, float* prepared,
 	int precision);
@@ -128,8 +134,8 @@ typedef struct nb200_conv_desc {
 	int ho, wo;                  /* result */
 } nb200_conv_desc;
 /* `scratch` is optional (NULL = none): nb200_blob_convolution_scratch_floats(desc) floats of device memory for what
- * the fast paths prepare once per call: the filter split for the tensor core (lo part / rounded copy, so that no CTA
- * converts its filter tiles), and for few-channel images (the 3-channel network stem) a copy of the image with its
+ * the fast paths prepare once per call: the filter split for the tensor core (lo part, fp16 halves or rounded copy, so that
+ * no CTA converts its filter tiles), and for few-channel images (the 3-channel network stem) a copy of the image with its
  * spatial padding and 4-channel pixels plus the filter widened to match; for convolutions with few output tiles
  * (small batches) also room for the partial results of a split K loop, which a finishing pass sums in a fixed order
  * (results do not vary from run to run).  The engine takes it from its block pool; without it the same result is
