@@ -1195,7 +1195,11 @@ int launch_bn(const ContractionParams& p0, int batch, cudaStream_t stream)
 FastDiv fast_div(long long d)
 {
 	FastDiv f = {};
-	while((1LL << f.shift) < d) ++f.shift;
+	if(d <= 1) { // most of a product's; the general form costs a 64-bit division per divisor and launch
+		f.mul = 1;
+		return f;
+	}
+	f.shift = 64 - __builtin_clzll(static_cast<unsigned long long>(d - 1));
 	f.mul = static_cast<uint32_t>(((1ULL << 32) * static_cast<unsigned long long>((1LL << f.shift) - d)) / static_cast<unsigned long long>(d) + 1);
 	return f;
 }
@@ -1214,10 +1218,10 @@ SplitFinish split_k(ContractionParams& p, long long numTiles, int numKb, int bat
 {
 	SplitFinish finish = {};
 	p.kSplits = 1;
+	if(p.splitScratch == nullptr || batch != 1 || numKb < 8) return finish;
 	const int sms = sm_count();
 	const long long slab = static_cast<long long>(p.M) * p.N;
-	if(numTiles * 2 <= sms && numKb >= 8 && p.c_vec && !p.accumulate && batch == 1 && p.ldc == p.N
-		&& p.splitScratch != nullptr && aligned16(p.splitScratch) && !(g_traceOptions & 32)) {
+	if(numTiles * 2 <= sms && p.c_vec && !p.accumulate && p.ldc == p.N && aligned16(p.splitScratch) && !(g_traceOptions & 32)) {
 		const long long room = sms / numTiles;
 		// at least four K blocks per part (measured: two is no better, eight is slower at batch 1)
 		for(int d = 2; d <= numKb / 4 && d <= room && d * slab <= p.splitScratchFloats; ++d) {
@@ -1320,7 +1324,8 @@ int balanced_tile_width(const ContractionParams& p, long long mTiles, int batch)
 	long long least = -1;
 	for(int i = 0; i < 4; ++i) {
 		const long long tiles = mTiles * ((p.N + widths[i] - 1) / widths[i]) * batch;
-		const long long total = (tiles + sms - 1) / sms * (stores[vec][i] + numKb * perBlock[vec][i]);
+		const long long waves = tiles <= sms ? 1 : (tiles + sms - 1) / sms;
+		const long long total = waves * (stores[vec][i] + numKb * perBlock[vec][i]);
 		if(least < 0 || total < least) { least = total; best = widths[i]; }
 	}
 	return best;
