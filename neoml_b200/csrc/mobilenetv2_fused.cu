@@ -68,22 +68,24 @@ __device__ __forceinline__ float lo_part(float v)
 	return v - __uint_as_float(__float_as_uint(v) & 0xffffe000u);
 }
 
-// ReLU (optionally with an upper threshold) and "no activation" as one clamp, or HSwish.  Which of the two is a template
-// parameter: the depthwise warps apply it to 72 + 32 values per tile, and as a choice at run time both were computed.
-// (64 x 56 x 56, 32 -> 192 -> 32: 150.7 -> 148.5 us with the tests of interior tiles left out as well; the tile's period is
-// still set by the tensor-memory reads, the A operand's stores and the barrier.)
+// ReLU (optionally with an upper threshold) and "no activation" as one clamp, or HSwish.  Whether a block has an HSwish at all is
+// a template parameter: the depthwise warps apply the activations to 72 + 32 values per tile, and as a choice at run time both
+// kinds are computed (64 x 56 x 56, 32 -> 192 -> 32, ReLU6: 150.7 -> 148.5 us with the tests of interior tiles left out as well;
+// the tile's period is still set by the tensor-memory reads, the A operand's stores and the barrier).
 template<bool HSWISH>
 struct Act {
+	bool hswish;
 	float lo, hi;
 	__device__ __forceinline__ float operator()(float v) const
 	{
-		return HSWISH ? v * fminf(fmaxf(v + 3.f, 0.f), 6.f) * (1.f / 6.f) : fminf(fmaxf(v, lo), hi);
+		return HSWISH && hswish ? v * fminf(fmaxf(v + 3.f, 0.f), 6.f) * (1.f / 6.f) : fminf(fmaxf(v, lo), hi);
 	}
 };
 template<bool HSWISH>
 __device__ __forceinline__ Act<HSWISH> make_act(int kind, float param)
 {
 	Act<HSWISH> a;
+	a.hswish = kind == NB200_ACT_HSWISH;
 	a.lo = kind == NB200_ACT_RELU ? 0.f : -__int_as_float(0x7f800000);
 	a.hi = kind == NB200_ACT_RELU && param > 0.f ? param : __int_as_float(0x7f800000);
 	return a;
@@ -123,7 +125,7 @@ __host__ __device__ inline SmemLayout smem_layout(int cExp, int cOut)
 	return l;
 }
 
-template<bool THREEX, bool HSWISH_EXP, bool HSWISH_DW>
+template<bool THREEX, bool HSWISH>
 __global__ void __launch_bounds__(THREADS, 1) mbv2_fused_kernel(const FusedParams p, const __grid_constant__ CUtensorMap mapX)
 {
 	extern __shared__ uint8_t smemRaw[];
@@ -191,8 +193,8 @@ __global__ void __launch_bounds__(THREADS, 1) mbv2_fused_kernel(const FusedParam
 	const uint32_t accProject = tmemBase + 4 * HALO_N;         // cOut columns; lanes 64..127 = the tile's 64 pixels
 	const uint32_t idescExpand = umma_idesc_tf32(128, HALO_N);
 	const uint32_t idescProject = umma_idesc_tf32(128, p.cOut);
-	const auto actExp = make_act<HSWISH_EXP>(p.actExp, p.actExpParam);
-	const auto actDw = make_act<HSWISH_DW>(p.actDw, p.actDwParam);
+	const auto actExp = make_act<HSWISH>(p.actExp, p.actExpParam);
+	const auto actDw = make_act<HSWISH>(p.actDw, p.actDwParam);
 
 	// Roles.  The lane quarter a warp may read (warp % 4) holds the 32 channels of chunk `combo`; a chunk has two
 	// depthwise warps, one per pair of output rows.  Quarters 2 and 3 exist only in the first 128-channel block: of
@@ -409,7 +411,7 @@ __global__ void __launch_bounds__(THREADS, 1) mbv2_fused_kernel(const FusedParam
 				}
 				tmem_ld_wait();
 				// The halo pixel's expanded value is zero outside the image.  A tile whose halo lies inside it (most tiles of a
-				// large image) runs the same arithmetic without the tests.
+				// large image) runs the same arithmetic without the tests (not with HSwish, whose two copies took 7 % longer).
 				auto depthwise = [&](auto inside) {
 					auto expanded = [&](uint32_t bits, int r, int hx) {
 						const float v = actExp(__uint_as_float(bits) + biasExp);
@@ -440,7 +442,7 @@ __global__ void __launch_bounds__(THREADS, 1) mbv2_fused_kernel(const FusedParam
 						}
 					}
 				};
-				if((rowBits[0] & rowBits[1] & rowBits[2] & rowBits[3]) == (1u << HW) - 1u) depthwise(Flag<true>());
+				if(!HSWISH && (rowBits[0] & rowBits[1] & rowBits[2] & rowBits[3]) == (1u << HW) - 1u) depthwise(Flag<true>());
 				else depthwise(Flag<false>());
 				// project(j-1) still reads the A tiles when this tile's arithmetic is done early: wait, then write
 				if(j > 0) {
@@ -509,22 +511,20 @@ __global__ void __launch_bounds__(THREADS, 1) mbv2_fused_kernel(const FusedParam
 	if(warp == 0) tmem_dealloc(tmemBase, TMEM_COLS);
 }
 
-template<bool THREEX, bool HSWISH_EXP, bool HSWISH_DW>
+template<bool THREEX, bool HSWISH>
 void launch_variant(const FusedParams& p, const CUtensorMap& map, int grid, size_t smemBytes, cudaStream_t stream)
 {
-	if(cudaFuncSetAttribute(mbv2_fused_kernel<THREEX, HSWISH_EXP, HSWISH_DW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+	if(cudaFuncSetAttribute(mbv2_fused_kernel<THREEX, HSWISH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
 		static_cast<int>(smemBytes)) == cudaSuccess) {
-		mbv2_fused_kernel<THREEX, HSWISH_EXP, HSWISH_DW><<<grid, THREADS, smemBytes, stream>>>(p, map);
+		mbv2_fused_kernel<THREEX, HSWISH><<<grid, THREADS, smemBytes, stream>>>(p, map);
 	}
 }
 
 template<bool THREEX>
-void launch_kind(const FusedParams& p, const CUtensorMap& map, bool hsExp, bool hsDw, int grid, size_t smemBytes, cudaStream_t stream)
+void launch_kind(const FusedParams& p, const CUtensorMap& map, bool hswish, int grid, size_t smemBytes, cudaStream_t stream)
 {
-	if(hsExp && hsDw) launch_variant<THREEX, true, true>(p, map, grid, smemBytes, stream);
-	else if(hsExp) launch_variant<THREEX, true, false>(p, map, grid, smemBytes, stream);
-	else if(hsDw) launch_variant<THREEX, false, true>(p, map, grid, smemBytes, stream);
-	else launch_variant<THREEX, false, false>(p, map, grid, smemBytes, stream);
+	if(hswish) launch_variant<THREEX, true>(p, map, grid, smemBytes, stream);
+	else launch_variant<THREEX, false>(p, map, grid, smemBytes, stream);
 }
 
 } // namespace
@@ -557,9 +557,9 @@ bool launch_mbv2_fused(void* stream, const nb200_mbv2_desc* d, const float* x, c
 	CUtensorMap map;
 	if(!make_image_box_map(&map, x, CIN, d->w, d->h, d->batch, CIN, HW, HH, 1)) return false;
 	const int grid = p.numTiles < sm_count() ? p.numTiles : sm_count();
-	const bool hsExp = d->act_exp == NB200_ACT_HSWISH, hsDw = d->act_dw == NB200_ACT_HSWISH;
-	if(precision == NB200_PREC_3XTF32) launch_kind<true>(p, map, hsExp, hsDw, grid, smemBytes, as_stream(stream));
-	else launch_kind<false>(p, map, hsExp, hsDw, grid, smemBytes, as_stream(stream));
+	const bool hswish = d->act_exp == NB200_ACT_HSWISH || d->act_dw == NB200_ACT_HSWISH;
+	if(precision == NB200_PREC_3XTF32) launch_kind<true>(p, map, hswish, grid, smemBytes, as_stream(stream));
+	else launch_kind<false>(p, map, hswish, grid, smemBytes, as_stream(stream));
 	count_launch(1);
 	*rc = check_launch();
 	return true;
