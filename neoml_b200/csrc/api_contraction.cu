@@ -241,6 +241,10 @@ void prepare_window_filter(void* stream, const nb200_conv_desc* d, const WindowP
 bool split_form_pays(const nb200_conv_desc* d, bool window)
 {
 	if(d->batch <= 0 || d->ho <= 0 || d->wo <= 0 || d->k <= 0) return false;
+	// row windows: filters of seven rows and more (K = 224) into whole 16-byte result rows; with five rows or odd filter counts the
+	// fp16 kernel's epilogue outlasts what its products save (16 x 100 x 32 x 3 by 100 x 5 x 5: 58.5 us with TF32 halves, 70.8;
+	// 32 x 87 x 34 x 3 by 195 x 7 x 7 / 2: 239.6, 264.9; by 192 filters 100.5, 77.1)
+	if(window && (d->r < 7 || d->k % 4 != 0)) return false;
 	const long long rows = static_cast<long long>(d->batch) * d->ho * d->wo;
 	return rows >= PREPARE_B_MIN_ROWS && split_form_pays(window ? static_cast<long long>(d->batch) * d->ho : (rows + 127) / 128,
 		d->k, window ? d->r * 32LL : static_cast<long long>(d->r) * d->s * d->c, 1);
