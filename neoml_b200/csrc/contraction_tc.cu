@@ -616,6 +616,9 @@ __global__ void __maxnreg__(128) contraction_tc_kernel(const ContractionParams p
 		const bool fastStore = vec && p.accumulate == 0 && p.act != NB200_ACT_HSWISH && p.act != NB200_ACT_SIGMOID_GATE;
 		const bool gateStore = vec && p.accumulate == 0 && p.act == NB200_ACT_SIGMOID_GATE;
 		const bool hswishStore = vec && p.accumulate == 0 && p.act == NB200_ACT_HSWISH;
+		// without a residual the element-wise stores, too, get a loop that tests for nothing but its bounds (60000 x 24 x 130: 54.5 us
+		// through the general one, 28.4)
+		const bool elementStore = p.accumulate == 0 && p.residual == nullptr && p.act != NB200_ACT_HSWISH && p.act != NB200_ACT_SIGMOID_GATE;
 		const bool clampOn = p.act == NB200_ACT_RELU;
 		const float actParam = p.act_param_device != nullptr ? __ldg(p.act_param_device) : p.act_param;
 		const float clampHi = actParam > 0.f ? actParam : __int_as_float(0x7f800000);
@@ -824,6 +827,20 @@ __global__ void __maxnreg__(128) contraction_tc_kernel(const ContractionParams p
 							float* dst = C + static_cast<size_t>(m) * p.ldc + n;
 							if(m < mEnd) {
 								asm volatile("st.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(o.x), "f"(o.y), "f"(o.z), "f"(o.w) : "memory");
+							}
+						}
+					} else if(elementStore) {
+						// result rows that are no whole 16-byte pieces (and columns beyond the last)
+						if(n < p.N)
+#pragma unroll
+						for(int i = 0; i < 4; ++i) {
+							const int m = rowBase + 8 * i + rowInGroup;
+							const float e[4] = { ov[i].x + bias4.x, ov[i].y + bias4.y, ov[i].z + bias4.z, ov[i].w + bias4.w };
+							float* dst = C + static_cast<size_t>(m) * p.ldc + n;
+#pragma unroll
+							for(int t = 0; t < 4; ++t) {
+								const float x = clampOn ? fminf(fmaxf(e[t], 0.f), clampHi) : e[t];
+								if(m < mEnd && n + t < p.N) dst[t] = x;
 							}
 						}
 					} else {
@@ -1306,26 +1323,34 @@ int contraction_tile_width(int n)
 }
 
 // The same where K is not split: the width whose waves over the SMs cost least.  A wave takes a time for its stores, which
-// grows with its columns, and one per K block, which hardly does (the copies and the conversion of A): in units of 10 ns,
-// fitted to 150 products of 3000 to 60000 rows, 64 to 1300 columns and K = 16 to 1024, every width timed.  Result rows that
-// are no whole 16-byte pieces are stored element by element, three to five times as slowly.  Slower than the best width by
-// 1.2 % on average at K <= 32, 0.2 to 1 % beyond, by 13 % at most; the least-padded width by 4 to 10 % at K <= 32, 10 to 15 %
-// at 64 and 128, 16 to 35 % beyond (1300 columns become 32 wide: 2048 x 1024 x 1300 86 us for 51), fixed costs per wave of
-// 100 : 90 : 80 : 62 by 6 to 13 % at K <= 32 (60000 x 24 x 130: 65.5 us, 53 here; 60000 x 32 x 576: 44.5, 38.3 here).
+// grows with its columns, and one per K block, which hardly does (the copies and the conversion of A); only their ratio
+// matters.  Fitted to 300 products of 3000 to 60000 rows, 33 to 1300 columns and K = 16 to 1024, every width timed.
+// Result rows that are no whole 16-byte pieces are stored element by element: by the fp16 kernel and with a residual or
+// other activations than ReLU three to five times as slowly, else twice.  Slower than the best width by 1 to 2 % on average,
+// 18 % at most (30 % in the fp16 kernel); the least-padded width by 4 to 10 % at K <= 32, 10 to 15 % at 64 and 128, 16 to 35 %
+// beyond (1300 columns become 32 wide: 2048 x 1024 x 1300 86 us for 51), fixed costs per wave of 100 : 90 : 80 : 62 by 6 to
+// 13 % at K <= 32 (60000 x 32 x 576: 44.5 us, 38.3 here).
 int balanced_tile_width(const ContractionParams& p, long long mTiles, int batch)
 {
 	const int widths[4] = { 128, 96, 64, 32 };
-	const long long stores[2][4] = { { 1225, 900, 580, 255 }, { 250, 172, 125, 86 } };
-	const long long perBlock[2][4] = { { 30, 30, 30, 30 }, { 45, 44, 43, 37 } };
-	const int vec = p.c_vec != 0 && p.accumulate == 0 ? 1 : 0;
+	enum { VEC = 0, ELEMENTS = 1, SLOW_ELEMENTS = 2 };
+	const long long stores[3][4] = { { 250, 172, 125, 86 }, { 1000, 646, 412, 132 }, { 1225, 900, 580, 255 } };
+	const long long perBlock[3][4] = { { 45, 44, 43, 37 }, { 150, 150, 150, 145 }, { 30, 30, 30, 30 } };
+	// an operand that is gathered takes longer per K block, whatever the width
+	const long long perGatheredBlock[3] = { 200, 800, 200 };
+	const bool gather = p.a_vec == 0 || p.b_vec == 0 || p.b_mode != B_ROWS || (p.a_mode == A_CONV_TAP && p.Cin % BK != 0);
+	const bool slow = p.bSplit != nullptr || p.residual != nullptr || p.accumulate != 0 || (p.act != NB200_ACT_NONE && p.act != NB200_ACT_RELU);
+	const int kind = p.c_vec != 0 && p.accumulate == 0 ? VEC : slow ? SLOW_ELEMENTS : ELEMENTS;
 	const long long numKb = (p.K + BK - 1) / BK;
+	// row windows: a tile is an output row, which may have far fewer than 128 positions to store
+	const int rows = p.a_mode == A_CONV_WINDOW && p.tileM > 0 && p.tileM < BM ? p.tileM : BM;
 	const int sms = sm_count();
 	int best = 128;
 	long long least = -1;
 	for(int i = 0; i < 4; ++i) {
 		const long long tiles = mTiles * ((p.N + widths[i] - 1) / widths[i]) * batch;
 		const long long waves = tiles <= sms ? 1 : (tiles + sms - 1) / sms;
-		const long long total = waves * (stores[vec][i] + numKb * perBlock[vec][i]);
+		const long long total = waves * (stores[kind][i] * rows / BM + numKb * (gather ? perGatheredBlock[kind] : perBlock[kind][i]));
 		if(least < 0 || total < least) { least = total; best = widths[i]; }
 	}
 	return best;
@@ -1338,7 +1363,8 @@ int launch_contraction_tc(const ContractionParams& p, int batch, cudaStream_t st
 	if(p.bSplit != nullptr) return (g_traceOptions & 16) ? NB200_EINVAL : launch_contraction_split(p, batch, stream);
 	// (with room for split K, a few-tile launch keeps the least-padded width: its parts fill the machine whatever the width)
 	const bool maySplit = p.splitScratch != nullptr && batch == 1 && p.K >= 8 * BK;
-	const long long mTiles = (p.M + BM - 1LL) / BM;
+	const int tileM = p.a_mode == A_CONV_WINDOW && p.tileM > 0 && p.tileM <= BM ? p.tileM : BM;
+	const long long mTiles = (p.M + tileM - 1LL) / tileM;
 	switch(maySplit ? contraction_tile_width(p.N) : balanced_tile_width(p, mTiles, batch)) {
 		case 32: return launch_bn<32>(p, batch, stream);
 		case 64: return launch_bn<64>(p, batch, stream);

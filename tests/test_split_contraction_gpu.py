@@ -218,9 +218,15 @@ def test_tile_widths(ops, m, k, n, precision):
     g.manual_seed(m)
     a, b = torch.empty(m, k, device="cuda").normal_(generator=g), torch.empty(n, k, device="cuda").normal_(generator=g)
     res = torch.empty(m, n, device="cuda").normal_(generator=g)
-    got = ops.MultiplyMatrixByTransposedMatrix(a, b, residual=res, precision=precision)
     # 8 products at a time; plain TF32 rounds both operands to 11 bits
-    assert worst(got, a, b, extra=res) < 2 * bound(k) + (2.0 ** -10 if precision else 0.0)
+    limit = 2 * bound(k) + (2.0 ** -10 if precision else 0.0)
+    got = ops.MultiplyMatrixByTransposedMatrix(a, b, residual=res, precision=precision)
+    assert worst(got, a, b, extra=res) < limit
+    bias = torch.empty(n, device="cuda").normal_(generator=g)
+    got = ops.MultiplyMatrixByTransposedMatrix(a, b, free_term=bias, precision=precision)
+    assert worst(got, a, b, extra=bias.expand(m, n)) < limit
+    clamped = ops.MultiplyMatrixByTransposedMatrix(a, b, free_term=bias, act=ops.ACT_RELU, act_param=2.5, precision=precision)
+    assert torch.equal(clamped, got.clamp(0.0, 2.5))
 
 
 @pytest.mark.parametrize("shape,k,r,stride,pad", [((5, 45, 47, 64), 70, 3, 1, 1), ((9, 40, 40, 160), 96, 1, 1, 0),
